@@ -83,6 +83,19 @@ __device__ __forceinline__ void tma_load_5d(void *dst, const CUtensorMap *tm, ui
         : "memory");
 }
 
+// One lane of a converged warp.  A loop of tcgen05.mma is to run under this
+// and not under lane == 0: the compiler then keeps the instruction's operands
+// in uniform registers, where a data-dependent branch makes it move each of
+// them there before every MMA.  256 MMAs of M = 128, K = 16 back to back, A in
+// TMEM: 110 cycles each under threadIdx.x == 0 whatever N up to 192; 43 at
+// N = 64, 59 at N = 96, 75 at N = 128 under elect.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+    return e != 0;
+}
+
 // ---- tcgen05 ---------------------------------------------------------------
 // Shared-memory matrix descriptor, K-major, no swizzle: 8-row x 16-byte core
 // matrices; rows of a core matrix 16 B apart; `lbo` = byte distance between

@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(256, 1) sur_conv_tc_kernel(const __grid_consta
     tc_fence_after();
     const uint32_t tmem = *tslot;
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0 && elect_one()) {
         // ---- producer: TMA loads of every item's nout + 2 input rows ----
         uint32_t g = 0;
         bool ok = true;
@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(256, 1) sur_conv_tc_kernel(const __grid_consta
         // every load has landed before the CTA exits
         for (uint32_t j = g > (uint32_t)kSurSlots ? g - kSurSlots : 0; j < g; j++)
             mbar_wait_bounded(&full[j % kSurSlots], (j / kSurSlots) & 1);
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1 && elect_one()) {
         // ---- MMA issuer ----
         const uint32_t wbase = smem_u32(wsm), sbase = smem_u32(slots);
         uint32_t g = 0, li = 0;
@@ -664,7 +664,7 @@ __global__ void __launch_bounds__(256, 1) sur_wgrad_tc_kernel(const __grid_const
     tc_fence_after();
     const uint32_t tmem = *tslot;
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0 && elect_one()) {
         // ---- producer: per item three gradient rows and one activation row ----
         uint32_t g = 0;
         bool ok = true;
@@ -686,7 +686,7 @@ __global__ void __launch_bounds__(256, 1) sur_wgrad_tc_kernel(const __grid_const
         if (!ok) atomicExch(a.err, GLSU_ERR_TIMEOUT);
         for (uint32_t j = g > (uint32_t)kWgStages ? g - kWgStages : 0; j < g; j++)
             mbar_wait_bounded(&full[j % kWgStages], (j / kWgStages) & 1);
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1 && elect_one()) {
         // ---- MMA issuer ----
         const uint32_t idesc = umma_idesc_bf16(128, 96) | (1u << 15) | (1u << 16);  // A and B MN-major
         uint32_t g = 0, acc = 0;
