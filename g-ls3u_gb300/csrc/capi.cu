@@ -300,6 +300,7 @@ extern "C" int glsu_wff_create(glsu_wff **out, int precision, int width, int hei
     if (rc == GLSU_OK) rc = h->plan.alloc_device();
     if (rc == GLSU_OK) rc = h->plan.upload_tables(h->stream);
     if (rc == GLSU_OK) rc = h->plan.make_tensor_map();
+    if (rc == GLSU_OK) rc = h->plan.init_tc();
     if (rc == GLSU_OK) rc = h->plan.init_colfft();
     if (rc == GLSU_OK) rc = h->plan.autotune(h->stream);
     if (rc == GLSU_OK && (cudaEventCreate(&h->ev0) != cudaSuccess || cudaEventCreate(&h->ev1) != cudaSuccess))
@@ -473,7 +474,7 @@ static int set_method(WffPlan &P, int method, cudaStream_t s)
     GLSU_CUDA_TRY(cudaStreamSynchronize(s));
     P.method = method;
     if (method == GLSU_METHOD_AUTO || method == GLSU_METHOD_TIMED) return P.autotune(s);
-    return GLSU_OK;
+    return P.ensure_colfft();
 }
 
 static void get_tuning(const WffPlan &P, glsu_wff_tuning *t)
@@ -504,7 +505,9 @@ extern "C" int glsu_wff_set_fft_plan(glsu_wff *h, int columns_per_cta, int radix
 {
     if (!h) return fail(GLSU_ERR_INVALID, "null handle");
     GLSU_CUDA_TRY(cudaStreamSynchronize(h->stream));
-    return h->plan.set_fft_plan(columns_per_cta, radix_order);
+    GLSU_TRY(h->plan.set_fft_plan(columns_per_cta, radix_order));
+    h->plan.fft_explicit = true;
+    return h->plan.ensure_colfft();
 }
 
 extern "C" int glsu_wff_set_fft_length(glsu_wff *h, int length)
@@ -512,7 +515,9 @@ extern "C" int glsu_wff_set_fft_length(glsu_wff *h, int length)
     if (!h) return fail(GLSU_ERR_INVALID, "null handle");
     if (h->plan.fft_L == 0) return fail(GLSU_ERR_UNSUPPORTED, "no shared-memory FFT plan for this handle");
     GLSU_CUDA_TRY(cudaStreamSynchronize(h->stream));
-    return h->plan.build_colfft(length);
+    GLSU_TRY(h->plan.build_colfft(length));
+    h->plan.fft_explicit = true;
+    return GLSU_OK;
 }
 
 extern "C" int glsu_wff_fft_lengths(const glsu_wff *h, int *lengths, int n)
@@ -583,6 +588,8 @@ extern "C" int glsu_dpra_create(glsu_dpra **out, int precision, const void *h_ph
     if (rc == GLSU_OK) rc = h->wff.alloc_device();
     if (rc == GLSU_OK) rc = h->wff.upload_tables(h->stream);
     if (rc == GLSU_OK) rc = h->wff.make_tensor_map();
+    h->wff.unit_input = true;  // exp(j dphi)
+    if (rc == GLSU_OK) rc = h->wff.init_tc();
     if (rc == GLSU_OK) rc = h->wff.init_colfft();
     if (rc == GLSU_OK) rc = h->wff.autotune(h->stream);
     const size_t N = (size_t)width * height;
@@ -1249,7 +1256,7 @@ static int batch_enqueue(glsu_dpra_batch *b, const std::vector<char> &active, co
     GLSU_TRY(batch_event(b, ne++, &fork));
     GLSU_CUDA_TRY(cudaEventRecord(fork, b->stream));
     // stage 1: least squares and row pass (and the direct column sweep)
-    std::map<int, std::vector<const WffPlan *>> classes;
+    std::map<std::pair<int, double>, std::vector<const WffPlan *>> classes;  // (FFT length, 0) or (-half size, sigma)
     for (size_t i = 0; i < b->h.size(); i++) {
         if (!active[i]) continue;
         glsu_dpra *h = b->h[i];
@@ -1257,13 +1264,14 @@ static int batch_enqueue(glsu_dpra_batch *b, const std::vector<char> &active, co
         GLSU_TRY(launch_dpra_ls(h->prec, img_type, in[i], h->d_phi[GLSU_PHI_REF], h->d_z, h->W, h->H, h->r,
                                 h->stream, h->ls_method, h->ls_tile));
         GLSU_TRY(h->wff.enqueue_pre(h->stream, h->d_z));
-        if (h->wff.use_colfft()) classes[h->wff.fft_L].push_back(&h->wff);
+        if (h->wff.use_tc()) classes[{-h->wff.sy, h->wff.p.sigma_y}].push_back(&h->wff);
+        else if (h->wff.use_colfft()) classes[{h->wff.fft_L, 0.0}].push_back(&h->wff);
         else GLSU_TRY(launch_column_sweep(h->wff, h->stream));
         GLSU_TRY(batch_event(b, ne++, &e));
         GLSU_CUDA_TRY(cudaEventRecord(e, h->stream));
         GLSU_CUDA_TRY(cudaStreamWaitEvent(b->stream, e, 0));
     }
-    // stage 2: the FFT column sweeps, one persistent launch per length
+    // stage 2: the column sweeps, one persistent launch per window (tensor cores) or FFT length
     cudaEvent_t pre = nullptr;
     GLSU_TRY(batch_event(b, ne++, &pre));
     GLSU_CUDA_TRY(cudaEventRecord(pre, b->stream));
@@ -1276,7 +1284,8 @@ static int batch_enqueue(glsu_dpra_batch *b, const std::vector<char> &active, co
         }
         cudaStream_t st = b->cls_stream[c++];
         GLSU_CUDA_TRY(cudaStreamWaitEvent(st, pre, 0));
-        GLSU_TRY(launch_colfft_batch(kv.second.data(), (int)kv.second.size(), st));
+        if (kv.first.first <= 0) GLSU_TRY(launch_tc_sweep(kv.second.data(), (int)kv.second.size(), st));
+        else GLSU_TRY(launch_colfft_batch(kv.second.data(), (int)kv.second.size(), st));
         GLSU_TRY(batch_event(b, ne++, &e));
         GLSU_CUDA_TRY(cudaEventRecord(e, st));
         GLSU_CUDA_TRY(cudaStreamWaitEvent(b->stream, e, 0));

@@ -184,6 +184,8 @@ struct WffPlan {
     void *d_tw = nullptr;           // fft_L twiddles e^{-2 pi i t / L}
     int init_colfft();
     int build_colfft(int L);  // tables for transform length L, default plan variant
+    int set_fft_len(int L);   // the length and its default variant; tables come with build_colfft
+    int ensure_colfft();      // the tables of the current length, where the sweep that runs needs them
     void release_colfft();
     // FFT plan variant: nc columns per CTA, radix order; GLSU_ERR_UNSUPPORTED
     // where it does not fit (the plan is then unchanged).
@@ -205,8 +207,26 @@ struct WffPlan {
     {
         return (method == GLSU_METHOD_AUTO || method == GLSU_METHOD_TIMED) ? auto_method : method;
     }
-    bool use_colfft() const { return fft_L > 0 && d_khat != nullptr && column_method() == GLSU_METHOD_FFT; }
+    bool use_colfft() const { return fft_L > 0 && column_method() == GLSU_METHOD_FFT; }
+
+    // Column sweep on the tensor cores (wff_tcsweep.cu): runs in the place of
+    // the FFT sweep wherever that is selected and no FFT length or plan was
+    // set by hand (or by timing).
+    bool fft_explicit = false;
+    bool unit_input = false;   // |f| <= 1 at every pixel (DPRA): the scale of R is a constant
+    void *d_tctaps = nullptr;  // B operand of the banded products, hi and lo FP16 parts
+    void *d_ey2 = nullptr;     // wy phasors of row pairs
+    float *d_kr = nullptr;     // [0] the power of two that R carries, [1] scratch
+    CUtensorMap tmT;           // d_R in row pairs: {4 pitch floats, (H + 1) / 2, nfx}
+    float tc_tscale = 1, tc_sum_gx = 1;
+    bool tc_supported() const;
+    int init_tc();
+    void release_tc();
+    bool use_tc() const { return use_colfft() && d_tctaps != nullptr && !fft_explicit; }
 };
+int launch_tc_scale(const WffPlan &P, const void *d_f, cudaStream_t s);
+int launch_tc_sweep(const WffPlan *const *plans, int n, cudaStream_t s);
+double tc_model_ms(const WffPlan &P);
 
 // The transform lengths the autotuner times for this plan (cheapest first).
 int fft_length_candidates(const WffPlan &P, int *out, int n);

@@ -65,7 +65,25 @@ int WffPlan::init_colfft()
     if (prec != GLSU_F32) return GLSU_OK;
     int L;
     if (length_candidates(H + 2 * sy, &L, 1) < 1) return GLSU_OK;  // taller than the longest plan: direct kernel
-    return build_colfft(L);
+    return set_fft_len(L);
+}
+
+int WffPlan::set_fft_len(int L)
+{
+    colfft::LenInfo li;
+    if (prec != GLSU_F32 || L < H + 2 * sy || !colfft::len_info(L, &li))
+        return fail(GLSU_ERR_UNSUPPORTED, "no compiled FFT plan of that length for this handle");
+    if (L != fft_L) release_colfft();
+    fft_L = L;
+    fft_nst = li.passes;
+    return set_fft_plan(li.ncol_default, 0);
+}
+
+// The tables take a few tenths of a second to compute, so a handle whose
+// sweep runs on the tensor cores or directly does without.
+int WffPlan::ensure_colfft()
+{
+    return (use_colfft() && !use_tc() && !d_khat) ? build_colfft(fft_L) : GLSU_OK;
 }
 
 // Tables of the FFT sweep for transform length L (replacing any others),
@@ -77,6 +95,7 @@ int WffPlan::build_colfft(int L)
     colfft::LenInfo li;
     if (prec != GLSU_F32 || L < H + 2 * sy || !colfft::len_info(L, &li))
         return fail(GLSU_ERR_UNSUPPORTED, "no compiled FFT plan of that length for this handle");
+    const int nc = (L == fft_L) ? fft_nc : li.ncol_default;
     release_colfft();
     std::vector<float> kh(2 * (size_t)nfy * L), tw(2 * (size_t)L);
     for (int k = 0; k < nfy; k++) {
@@ -105,7 +124,7 @@ int WffPlan::build_colfft(int L)
     GLSU_CUDA_TRY(cudaMemcpy(d_tw, tw.data(), tw.size() * sizeof(float), cudaMemcpyHostToDevice));
     fft_L = L;
     fft_nst = li.passes;
-    return set_fft_plan(li.ncol_default, 0);
+    return set_fft_plan(nc, 0);
 }
 
 int fft_length_candidates(const WffPlan &P, int *out, int n)
@@ -136,6 +155,7 @@ void WffPlan::release_colfft()
 
 int launch_colfft(const WffPlan &P, cudaStream_t s)
 {
+    if (!P.d_khat) return fail(GLSU_ERR_INVALID, "column FFT sweep without its tables");
     const int ngroups = P.pitch / P.fft_nc;
     int grid_x = ngroups;
     const int2 *list = nullptr;
@@ -178,7 +198,7 @@ int launch_colfft_batch(const WffPlan *const *plans, int n, cudaStream_t s)
         int nitems = 0;
         for (int k = 0; k < m; k++) {
             const WffPlan &P = *plans[i0 + k];
-            if (P.fft_L != L || !P.use_colfft() || P.prec != GLSU_F32 || P.pitch % nc != 0)
+            if (P.fft_L != L || !P.use_colfft() || !P.d_khat || P.prec != GLSU_F32 || P.pitch % nc != 0)
                 return fail(GLSU_ERR_INVALID, "batched column sweep: plans of one FFT length only");
             const double N = 1.0 / P.inv_norm;
             colfft::BatchSeq &q = tab.seq[k];
@@ -217,7 +237,7 @@ int launch_colfft_batch(const WffPlan *const *plans, int n, cudaStream_t s)
 //
 // Timed search.  Candidates: the direct column kernel, and the FFT sweep at
 // the two shortest compiled transform lengths, then, at the faster length,
-// with the other compiled CTA width.  Each is launched once (warm-up), then
+// with the other compiled CTA width, and the tensor-core sweep.  Each is launched once (warm-up), then
 // twice between CUDA events on the plan's own buffers; the kernels have no
 // data-dependent control flow, so the buffers' contents do not matter.  The
 // FFT is taken only when at least 10% faster than the direct kernel, so
@@ -231,6 +251,7 @@ struct TuneKey {
 struct TuneResult {
     int method, L, nc, order;
     float ms_direct, ms_fft;
+    bool tc;  // the tensor-core sweep was the fastest but for the direct kernel
 };
 std::mutex g_tune_mu;
 std::map<TuneKey, TuneResult> g_tune;
@@ -258,6 +279,7 @@ double WffPlan::model_ms(int m) const
 {
     if (m == GLSU_METHOD_FFT) {
         if (fft_L == 0) return 1e30;
+        if (d_tctaps) return tc_model_ms(*this);
         const double units = (double)pitch * nfx * fft_L * (fft_nst * (2.0 * nfy + 2.0) + kModelFftColumnUnits);
         return units / kModelFftRate * 1e3 + kModelLaunchMs;
     }
@@ -273,16 +295,14 @@ double WffPlan::model_ms(int m) const
 int WffPlan::choose_by_model()
 {
     auto_method = GLSU_METHOD_DIRECT;
-    if (prec != GLSU_F32 || fft_L == 0 || d_khat == nullptr) return GLSU_OK;
+    if (prec != GLSU_F32 || fft_L == 0) return GLSU_OK;
     int L;
-    if (length_candidates(H + 2 * sy, &L, 1) == 1 && L != fft_L) GLSU_TRY(build_colfft(L));
-    colfft::LenInfo li;
-    colfft::len_info(fft_L, &li);
-    GLSU_TRY(set_fft_plan(li.ncol_default, 0));
+    if (length_candidates(H + 2 * sy, &L, 1) == 1) GLSU_TRY(set_fft_len(L));
+    fft_explicit = false;
     tune_ms_direct = (float)model_ms(GLSU_METHOD_DIRECT);
     tune_ms_fft = (float)model_ms(GLSU_METHOD_FFT);
     if (tune_ms_fft < 0.9f * tune_ms_direct) auto_method = GLSU_METHOD_FFT;
-    return GLSU_OK;
+    return ensure_colfft();
 }
 
 int WffPlan::autotune(cudaStream_t s)
@@ -291,7 +311,7 @@ int WffPlan::autotune(cudaStream_t s)
     timed = false;
     auto_method = GLSU_METHOD_DIRECT;
     tune_ms_direct = tune_ms_fft = 0;
-    if (prec != GLSU_F32 || fft_L == 0 || d_khat == nullptr) return GLSU_OK;
+    if (prec != GLSU_F32 || fft_L == 0) return GLSU_OK;
     const char *env = std::getenv("GLSU_AUTOTUNE");
     if (env && env[0] == '0') return GLSU_OK;
     const bool want_timing = method == GLSU_METHOD_TIMED || (env && std::strcmp(env, "time") == 0);
@@ -319,9 +339,12 @@ int WffPlan::autotune(cudaStream_t s)
                 rc = fail(GLSU_ERR_CUDA, "timing a column-sweep candidate failed");
             *ms *= 0.5f;
         };
-        TuneResult r{GLSU_METHOD_DIRECT, fft_L, fft_nc, fft_order, 0.f, 0.f};
+        TuneResult r{GLSU_METHOD_DIRECT, fft_L, fft_nc, fft_order, 0.f, 0.f, false};
         time_it(GLSU_METHOD_DIRECT, &r.ms_direct);
-        float best = -1.f;
+        float best = -1.f, tc = -1.f;
+        fft_explicit = false;
+        if (rc == GLSU_OK && d_tctaps) time_it(GLSU_METHOD_FFT, &tc);
+        fft_explicit = true;
         int lens[2];
         const int nl = length_candidates(H + 2 * sy, lens, 2);
         for (int j = 0; j < nl && rc == GLSU_OK; j++) {
@@ -349,6 +372,10 @@ int WffPlan::autotune(cudaStream_t s)
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
         if (rc != GLSU_OK) return rc;
+        if (tc > 0 && (best < 0 || tc < best)) {
+            r.tc = true;
+            best = tc;
+        }
         r.ms_fft = best;
         if (best > 0 && best < 0.9f * r.ms_direct) r.method = GLSU_METHOD_FFT;
         it = g_tune.emplace(key, r).first;
@@ -357,8 +384,10 @@ int WffPlan::autotune(cudaStream_t s)
     auto_method = r.method;
     tune_ms_direct = r.ms_direct;
     tune_ms_fft = r.ms_fft;
-    if (r.L != fft_L) GLSU_TRY(build_colfft(r.L));
-    return set_fft_plan(r.nc, r.order);
+    if (r.L != fft_L) GLSU_TRY(set_fft_len(r.L));
+    fft_explicit = !r.tc;
+    GLSU_TRY(set_fft_plan(r.nc, r.order));
+    return ensure_colfft();
 }
 
 }  // namespace glsu

@@ -77,10 +77,13 @@ template <typename T, int S> struct ColGeom {
 // ---------------------------------------------------------------------------
 // A: row pass with demodulation
 // ---------------------------------------------------------------------------
-template <typename T, int S>
+// PACK: the planes of the tensor-core sweep, rows in pairs (re, re', im, im')
+// and scaled by *kr, a power of two.
+template <typename T, int S, bool PACK>
 __global__ void __launch_bounds__(256) wff_rows_demod_kernel(const C2<T> *__restrict__ f, int W, int H,
                                                              int pitch, const C2<T> *__restrict__ ex, int nfx,
-                                                             C2<T> *__restrict__ R, Taps<T, S> gx, TileMask tm)
+                                                             C2<T> *__restrict__ R, Taps<T, S> gx, TileMask tm,
+                                                             const T *__restrict__ kr)
 {
     using G = RowGeom<T, S>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -131,6 +134,19 @@ __global__ void __launch_bounds__(256) wff_rows_demod_kernel(const C2<T> *__rest
             ot[lane * G::OUT_STRIDE + w * kRowK + k] = (gxx < W) ? mk<T>(ar[k], ai[k]) : mk<T>(0, 0);
         }
         __syncthreads();
+        if constexpr (PACK) {
+            const int pairs = (H + 1) / 2;
+            const T sc = *kr;
+            float4 *Rp = reinterpret_cast<float4 *>(R) + (size_t)i * pairs * pitch;
+            for (int e = tid; e < kRowTileRows / 2 * kRowTileCols; e += 256) {
+                const int r = e / kRowTileCols, c = e - r * kRowTileCols;
+                if (y0 / 2 + r >= pairs) break;
+                const C2<T> a = ot[2 * r * G::OUT_STRIDE + c], b = ot[(2 * r + 1) * G::OUT_STRIDE + c];
+                Rp[(size_t)(y0 / 2 + r) * pitch + x0 + c] = make_float4(a.x * sc, b.x * sc, a.y * sc, b.y * sc);
+            }
+            __syncthreads();
+            continue;
+        }
         C2<T> *Ri = R + i * plane;
         for (int e = tid; e < kRowTileRows * kRowTileCols; e += 256) {
             const int r = e / kRowTileCols, c = e - r * kRowTileCols;
@@ -563,11 +579,13 @@ int WffPlan::alloc_device()
     if (cudaMalloc(&d_ex, exn * cs) != cudaSuccess || cudaMalloc(&d_ey, eyn * cs) != cudaSuccess)
         return fail(GLSU_ERR_ALLOC, "cudaMalloc of phasor tables failed");
     if (!external_scratch) {
-        if (cudaMalloc(&d_R, (size_t)nfx * plane_bytes()) != cudaSuccess ||
+        // the tensor-core sweep keeps R in pairs of rows
+        const size_t r_bytes = (size_t)nfx * (plane_bytes() + (H & 1) * pitch * cs);
+        if (cudaMalloc(&d_R, r_bytes) != cudaSuccess ||
             cudaMalloc(&d_C, (size_t)nfx * plane_bytes()) != cudaSuccess)
             return fail(GLSU_ERR_ALLOC, "cudaMalloc of WFF2 planes failed");
         // defined contents: a tile-masked run reads planes it did not write
-        GLSU_CUDA_TRY(cudaMemset(d_R, 0, (size_t)nfx * plane_bytes()));
+        GLSU_CUDA_TRY(cudaMemset(d_R, 0, r_bytes));
         GLSU_CUDA_TRY(cudaMemset(d_C, 0, (size_t)nfx * plane_bytes()));
         if (cudaMalloc(&d_thr, sizeof(double)) != cudaSuccess ||
             cudaMalloc((void **)&d_part, sizeof(double) * kThrBlocks) != cudaSuccess ||
@@ -661,6 +679,7 @@ int WffPlan::alloc_tile_list()
 void WffPlan::release()
 {
     release_colfft();
+    release_tc();
     cudaFree(d_ex);
     cudaFree(d_ey);
     cudaFree(d_list);
@@ -708,17 +727,29 @@ static TileMask with_margins(TileMask m, int my, int mx)
     return m;
 }
 
+template <typename T, int S, bool PACK>
+static int launch_rows_demod_t(const WffPlan &P, const void *d_f, cudaStream_t s)
+{
+    using G = RowGeom<T, S>;
+    GLSU_TRY(raise_smem_limit((const void *)wff_rows_demod_kernel<T, S, PACK>, (int)G::SMEM));
+    dim3 grid(P.pitch / kRowTileCols, (P.H + kRowTileRows - 1) / kRowTileRows);
+    wff_rows_demod_kernel<T, S, PACK><<<grid, 256, G::SMEM, s>>>(
+        (const C2<T> *)d_f, P.W, P.H, P.pitch, (const C2<T> *)P.d_ex, P.nfx, (C2<T> *)P.d_R,
+        make_taps<T, S>(P.gx, P.sx, 1.0), with_margins(P.mask, 2 * P.sy, P.sx), (const T *)P.d_kr);
+    GLSU_CUDA_TRY(cudaGetLastError());
+    return GLSU_OK;
+}
+
 template <typename T, int S>
 static int launch_rows_demod(const WffPlan &P, const void *d_f, cudaStream_t s)
 {
-    using G = RowGeom<T, S>;
-    GLSU_TRY(raise_smem_limit((const void *)wff_rows_demod_kernel<T, S>, (int)G::SMEM));
-    dim3 grid(P.pitch / kRowTileCols, (P.H + kRowTileRows - 1) / kRowTileRows);
-    wff_rows_demod_kernel<T, S><<<grid, 256, G::SMEM, s>>>(
-        (const C2<T> *)d_f, P.W, P.H, P.pitch, (const C2<T> *)P.d_ex, P.nfx, (C2<T> *)P.d_R,
-        make_taps<T, S>(P.gx, P.sx, 1.0), with_margins(P.mask, 2 * P.sy, P.sx));
-    GLSU_CUDA_TRY(cudaGetLastError());
-    return GLSU_OK;
+    if constexpr (sizeof(T) == 4) {
+        if (P.use_tc()) {
+            if (!P.unit_input) GLSU_TRY(launch_tc_scale(P, d_f, s));
+            return launch_rows_demod_t<T, S, true>(P, d_f, s);
+        }
+    }
+    return launch_rows_demod_t<T, S, false>(P, d_f, s);
 }
 
 int WffPlan::enqueue_rows(cudaStream_t s, const void *d_f)
@@ -778,6 +809,10 @@ static int launch_final(const WffPlan &P, void *d_out, const void *phiref, const
 
 template <typename T> static int launch_cols_any(WffPlan &P, cudaStream_t s)
 {
+    if (sizeof(T) == 4 && P.use_tc()) {
+        const WffPlan *one = &P;
+        return launch_tc_sweep(&one, 1, s);
+    }
     if (sizeof(T) == 4 && P.use_colfft()) return launch_colfft(P, s);
     switch (P.syi) {
     case 12: return launch_cols<T, 12>(P, s);

@@ -1,0 +1,888 @@
+// wff_tcsweep.cu -- WFF2 column sweep on the tensor cores (FP32 form).
+//
+// The demodulated form of the sweep: for one x-frequency plane R and every wy
+//     U = (R e^{-j wy y}) (*)_y g,   T = U . [ |U| >= thr N ],
+//     C += e^{+j wy y} (T (*)_y g)
+// with g the real, truncated window of 2s+1 taps.  Each of the two
+// convolutions is a banded Toeplitz product.  The image columns are the M
+// rows of the MMA (64 columns, real and imaginary parts in lanes of their
+// own: M = 128), 16 image rows are its K, and the N outputs they reach --
+// 2s + 16, rounded up to a multiple of 16 -- its N.  The B operand is one
+// constant block B[n][j] = g(n - j - s) for every K step; the accumulator
+// window of a step starts 16 TMEM columns after that of the step before.
+//
+// FP32 in 11-bit operands: each value and each tap is split into two FP16
+// parts, x = hi + lo with |x - hi - lo| <= 2^-24 |x|, and a K step is three
+// MMAs, lo.hi + hi.lo + hi.hi, accumulated in FP32 (the dropped lo.lo is
+// 2^-24 of the product).  Powers of two keep both parts in FP16's normal
+// range: R is written by the row pass scaled to at most 2^15 (d_kr), the
+// taps by 2^6, T by tscale to at most 2^15.
+//
+// One CTA of seven warpgroups per SM walks a list of (plane, 64 columns, Rw
+// rows) tiles; the tile of R (Rw + 4s rows) stays in shared memory for all
+// wy.  Per 32 rows (two K steps):
+//   A  (2 x 4 warps)  R . e^{-j wy y}, split, tcgen05.st into an A1 slot
+//   M  (2 warps)      pass 1: A1 x B into U; pass 2: A2 x B into C
+//   B  (2 x 4 warps)  U from TMEM, threshold, split, into an A2 slot
+//   C  (2 x 4 warps)  finished rows from TMEM, times e^{+j wy y}, into registers
+// The operands never pass through shared memory: tcgen05.ld .16x256b and
+// tcgen05.st .16x128b give a thread the same image column and the same rows
+// on both sides, real part in lane i and imaginary in lane i + 8.
+//
+// TMEM holds all of a wy's rows of U and C (24 blocks of 16 columns) beside
+// the operand slots; the windows are cut to the blocks in which a needed row
+// lies.  A drained block is refilled with zeros, so every MMA accumulates, and
+// each accumulator sees the same K steps in the same order whatever the tile:
+// a row's bits do not depend on the tile height, the batch or a tile mask.
+//
+// Bound: instruction issue.  At 1024^2, sigma 10, 21 x 21 frequencies the sweep
+// takes 1.33 ms (the FFT sweep 3.18): 2.8 instructions a clock per SM, about
+// 170 per 16 x 64 block, wy and pass for the splitting and thresholding, a
+// quarter of them waiting.  Its MMAs alone would take 0.5 ms (N/2 cycles each at
+// M = 128, K = 16, A in TMEM); the DRAM is at 3%.
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+#include <type_traits>
+#include <vector>
+
+#include <cuda_fp16.h>
+
+#include "glsu_internal.cuh"
+#include "ptx_sm103.cuh"
+
+namespace glsu {
+namespace {
+
+constexpr int kBlocks = 24;       // blocks of 16 TMEM columns for the accumulators U and C
+constexpr int kCols = 64;         // image columns per CTA
+constexpr int kChunkRows = 64;    // rows of R per TMA chunk
+constexpr int kMaxChunks = 6;     // 384 rows of R in shared memory
+constexpr int kPhRing = 4;        // wy phasor tables in flight
+constexpr int kPhPairs = kMaxChunks * kChunkRows / 2;
+constexpr int kPairs = 8;         // pairs of blocks of either
+constexpr int kMaxTcHalf = 48;    // half-sizes: beyond, the truncation leaves more error than the FFT sweep has
+constexpr int kMaxN = 112;
+static_assert(16 * kBlocks + 2 * 2 * 32 <= 512, "TMEM columns");
+constexpr int kChunkBytes = kChunkRows * kCols * 8;
+constexpr int kPhBytes = kPhPairs * 16;
+constexpr int kMaxTapBytes = 2 * kMaxN * 32;  // hi and lo B operands
+constexpr int kTapShift = 6;                // taps scaled by 2^6
+// The tensor core's FP32 accumulation truncates: a pass of half-size s, 3
+// MMAs for each of about (2s + 16)/16 steps, comes out smaller by 0.6 to
+// 1.0e-8 s (half-sizes 6 to 48, fields of two sizes, against 64 bits), the
+// same for every row.  Threshold and output scale take the mean of it out:
+// the error against 64 bits at sigma 10 goes from 5.9e-7 to 1.4e-7 of the
+// output's norm, that of the FFT sweep.
+constexpr double kShrink = 0.82e-8;
+constexpr int kSmem = kMaxChunks * kChunkBytes + kPhRing * kPhBytes + kMaxTapBytes + 768 + 1024;
+static_assert(kSmem <= 227 * 1024, "column tile exceeds shared memory");
+
+// One sequence of the sweep.
+struct TcSeq {
+    CUtensorMap tm;      // R: {4 pitch floats, row pairs, planes}
+    const float4 *ey2;   // phasors of row pairs, [nfy][eys2], kTcPad pairs of padding in front
+    float2 *C;
+    const float *thr;
+    const float *kr;     // scale that R carries
+    int H, W, pitch, nfy, eys2, ncg, nty, item0;
+    float thr_mul, out_mul;
+};
+template <int NS> struct TcTable {
+    TcSeq seq[NS];
+};
+constexpr int kTcPad = 64;  // row pairs of padding in front of a phasor table
+
+// Geometry of one tile.  R row of pass-1 step q: ra + 16 q; U row of block p:
+// ra - s + 16 p; C row of block p: y0 + 16 (p - m).
+struct TcTile {
+    int plane, x0, y0, ra, q0, q1, p0, p1, nc;
+};
+
+__device__ __forceinline__ int fdiv16(int v) { return v >> 4; }  // floor
+
+__device__ __forceinline__ TcTile tc_tile(const TcSeq &q, int plane, int g, int ty, int s, int m, int rw)
+{
+    TcTile t;
+    t.plane = plane;
+    t.x0 = g * kCols;
+    t.y0 = ty * rw;
+    t.ra = t.y0 + 2 * s - 16 * m;
+    const int y1 = min(t.y0 + rw, q.H);
+    t.q0 = fdiv16(max(0, t.y0 - 2 * s) - t.ra);
+    t.q1 = fdiv16(min(q.H, y1 + 2 * s) - t.ra + 15);
+    t.p0 = fdiv16(max(0, t.y0 - s) - t.ra + s);
+    t.p1 = fdiv16(min(q.H, y1 + s) - t.ra + s + 15);
+    t.nc = (y1 - t.y0 + 15) >> 4;
+    return t;
+}
+
+// The three products of one K step (A hi at TMEM column a, lo at a + 8) into
+// the accumulators at d.  One asm statement with its own elect, in code that a
+// whole warp walks with warp-uniform operands: 3 MMAs with a wait before them
+// then issue in 190 cycles; with an elected thread walking the same loop it
+// is 305, most of it moving operands into uniform registers.
+__device__ __forceinline__ void umma_step(uint32_t d, uint32_t a, uint64_t bhi, uint64_t blo, uint32_t idesc)
+{
+    asm volatile(
+        "{\n\t.reg .pred p, e;\n\t.reg .b32 alo;\n\t"
+        "elect.sync _|e, 0xffffffff;\n\tsetp.ne.b32 p, 1, 0;\n\tadd.u32 alo, %1, 8;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [alo], %2, %4, p;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %3, %4, p;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %4, p;\n\t}" ::"r"(d),
+        "r"(a), "l"(bhi), "l"(blo), "r"(idesc)
+        : "memory");
+}
+// The same by a whole warp: arrive on bar when the MMAs that its elected thread issued have completed.
+__device__ __forceinline__ void umma_commit_warp(uint64_t *bar)
+{
+    asm volatile(
+        "{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
+        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar))
+        : "memory");
+}
+
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar)
+{
+    asm volatile(
+        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
+        "l"(src), "r"(bytes), "r"(smem_u32(bar))
+        : "memory");
+}
+
+// 16 lanes x 16 columns: r[4j + {0,1}] rows (lanes) t/4, columns 8j + 2(t%4) + {0,1}; r[4j + {2,3}] lane t/4 + 8.
+__device__ __forceinline__ void tmem_ld_16x256b_x2(uint32_t a, float *r)
+{
+    uint32_t u[8];
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7])
+                 : "r"(a));
+#pragma unroll
+    for (int i = 0; i < 8; i++) r[i] = __uint_as_float(u[i]);
+}
+// 16 lanes x 16 columns: r[2j] lane t/4, column 4j + t%4; r[2j + 1] lane t/4 + 8.
+__device__ __forceinline__ void tmem_st_16x128b_x4(uint32_t a, const uint32_t *r)
+{
+    asm volatile("tcgen05.st.sync.aligned.16x128b.x4.b32 [%8], {%0,%1,%2,%3,%4,%5,%6,%7};" ::"r"(r[0]), "r"(r[1]),
+                 "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(a)
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_zero16(uint32_t a)
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(a),
+                 "r"(0)
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// The loaded registers may be read only after the wait: tie them to it.
+__device__ __forceinline__ void tie8(float *r)
+{
+    asm volatile("" : "+f"(r[0]), "+f"(r[1]), "+f"(r[2]), "+f"(r[3]), "+f"(r[4]), "+f"(r[5]), "+f"(r[6]), "+f"(r[7]));
+}
+
+template <int N> __device__ __forceinline__ void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+
+// v = (v.x, v.y) as FP16 pairs hi and lo (v.x in the lower half)
+__device__ __forceinline__ void split2(float2 v, uint32_t &hi, uint32_t &lo)
+{
+    const __half2 h = __floats2half2_rn(v.x, v.y);
+    const float2 hf = __half22float2(h);
+    const float2 d = __ffma2_rn(hf, make_float2(-1.f, -1.f), v);
+    const __half2 l = __floats2half2_rn(d.x, d.y);
+    hi = *reinterpret_cast<const uint32_t *>(&h);
+    lo = *reinterpret_cast<const uint32_t *>(&l);
+}
+
+struct TcBars {
+    uint64_t rfull[kMaxChunks], rfree[kMaxChunks], phfull[kPhRing], phfree[kPhRing];
+    uint64_t a1full[2], a1free[2], a2full[2], a2free[2];
+    uint64_t ufull[kPairs], ufree[kPairs], cfull[kPairs], cfree[kPairs];  // per pair of blocks
+    uint64_t drain;
+    uint32_t tmem;
+};
+static_assert(sizeof(TcBars) <= 768, "barriers");
+
+// The value of lane 0, which the compiler then knows to be the warp's.
+__device__ __forceinline__ int uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
+
+// Wait, once the phase is not there yet with the bounded wait.  After a
+// timeout (ok false) waits return at once: the roles then run to their ends,
+// within their buffers, and the results are not used.
+__device__ __forceinline__ void wait_ok(uint64_t *bar, uint32_t parity, bool &ok)
+{
+    if (ok && !mbar_try_wait(bar, parity)) ok = mbar_wait_bounded(bar, parity);
+}
+
+// The same with a warp-uniform verdict.
+__device__ __forceinline__ void warp_wait(uint64_t *bar, uint32_t parity, bool &ok)
+{
+    if (!ok) return;
+    bool w = mbar_try_wait(bar, parity);
+    if (!w) w = mbar_wait_bounded(bar, parity);
+    ok = __all_sync(0xffffffffu, w);
+}
+
+// Seven warpgroups: loads and MMAs, two A, two B, two C.  A tile is RB pairs of
+// 16-row blocks.  RM, RA, RT, RC: registers a thread of each kind keeps of the
+// 72 at launch; the shares sum to the launch's.
+template <int RB_, int RM_, int RA_, int RT_, int RC_> struct TcCfg {
+    static constexpr int RB = RB_, RM = RM_, RA = RA_, RT = RT_, RC = RC_;
+    static_assert(RM + 2 * (RA + RT + RC) <= 7 * 72, "register shares");
+};
+constexpr int kThreads = 7 * 128;
+
+// Walks the CTA's items: fills t and the sequence index; false past the end.
+template <int NS>
+__device__ __forceinline__ int tc_item(const TcTable<NS> &tab, int nseq, int item, const int2 *list, int listn, int s,
+                                       int m, int rw, TcTile &t)
+{
+    int k = 0;
+    if (NS > 1) {
+        int hi = nseq - 1;  // the last sequence with item0 <= item
+        while (k < hi) {
+            const int mid = (k + hi + 1) >> 1;
+            if (tab.seq[mid].item0 <= item) k = mid;
+            else hi = mid - 1;
+        }
+    }
+    const TcSeq &q = tab.seq[k];
+    int local = item - q.item0;
+    if (list) {
+        const int2 e = list[local % listn];
+        t = tc_tile(q, local / listn, e.x, e.y, s, m, rw);
+    } else {
+        const int g = local % q.ncg;
+        local /= q.ncg;
+        t = tc_tile(q, local / q.nty, g, local % q.nty, s, m, rw);
+    }
+    return k;
+}
+
+template <class Cfg, int NS>
+__global__ void __launch_bounds__(kThreads, 1)
+    wff_tc_kernel(const __grid_constant__ TcTable<NS> tab, int nseq, int nitems_full, int s, int m, int N, float tscale,
+                  const uint4 *__restrict__ taps, int *__restrict__ err, const int2 *__restrict__ list,
+                  const int *__restrict__ list_count)
+{
+    constexpr int RB = Cfg::RB, RW = 32 * RB;
+    extern __shared__ unsigned char sm_raw[];
+    unsigned char *sm = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(sm_raw) + 1023) & ~(uintptr_t)1023);
+    unsigned char *Rs = sm;
+    float4 *ph = reinterpret_cast<float4 *>(Rs + kMaxChunks * kChunkBytes);
+    unsigned char *tb = reinterpret_cast<unsigned char *>(ph + kPhRing * kPhPairs);
+    TcBars &bar = *reinterpret_cast<TcBars *>(tb + kMaxTapBytes);
+
+    // warp-uniform to the compiler too: the operands of the tcgen05 instructions derive from it
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31, wg = warp >> 2, w4 = warp & 3;
+    const int nchunks = (RW + 16 * m + kChunkRows - 1) / kChunkRows;
+    int nitems = nitems_full, listn = 0;
+    if (list) {
+        listn = *list_count;
+        nitems = nitems_full * listn;  // nitems_full planes
+    }
+    if ((int)blockIdx.x >= nitems) return;  // uniform, before any barrier or allocation
+
+    if (tid == 0) {
+        for (int i = 0; i < kMaxChunks; i++) {
+            mbar_init(&bar.rfull[i], 1);
+            mbar_init(&bar.rfree[i], 8);
+        }
+        for (int i = 0; i < kPhRing; i++) {
+            mbar_init(&bar.phfull[i], 1);
+            mbar_init(&bar.phfree[i], 16);
+        }
+        for (int i = 0; i < 2; i++) {
+            mbar_init(&bar.a1full[i], 4);
+            mbar_init(&bar.a1free[i], 1);
+            mbar_init(&bar.a2full[i], 4);
+            mbar_init(&bar.a2free[i], 1);
+        }
+        for (int i = 0; i < kPairs; i++) {
+            mbar_init(&bar.ufull[i], 1);
+            mbar_init(&bar.ufree[i], 4);
+            mbar_init(&bar.cfull[i], 1);
+            mbar_init(&bar.cfree[i], 8);
+        }
+        mbar_init(&bar.drain, 2);
+        fence_mbar_init();
+    }
+    if (warp == 0) tmem_alloc(&bar.tmem, 512);
+    for (int e = tid; e < N * 4; e += kThreads) reinterpret_cast<uint4 *>(tb)[e] = taps[e];  // hi, then lo
+    fence_proxy_async_smem();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, bar.tmem, 0);
+    const uint32_t tU = tmem, tC = tmem + 16 * (kBlocks - 2 * RB), tA1 = tmem + 16 * kBlocks, tA2 = tA1 + 64;
+    if (wg == 1) {
+        for (int c = 0; c < 16 * kBlocks; c += 16) tmem_zero16(tmem + c + ((uint32_t)w4 << 21));
+        tmem_wait_st();
+        tc_fence_before();
+    }
+    __syncthreads();
+    tc_fence_after();
+
+    // fragment coordinates: first row pair within a block, image column within 8
+    const int frow = lane & 3, fi = lane >> 2, fcol = (fi >> 1) | ((fi & 1) << 2);
+    const uint32_t lanes = (uint32_t)w4 << 21;
+    bool ok = true;
+
+    if (wg == 0) {
+        reg_dec<Cfg::RM>();
+        if (warp == 1 && elect_one()) {
+            // ---- loads: R chunks of each tile, one phasor table per wy ----
+            uint32_t nk = 0, nit = 0;
+            for (int item = blockIdx.x; item < nitems; item += gridDim.x, nit++) {
+                TcTile t;
+                const TcSeq &q = tab.seq[tc_item<NS>(tab, nseq, item, list, listn, s, m, RW, t)];
+                for (int ch = 0; ch < nchunks && ok; ch++) {
+                    if (nit > 0) wait_ok(&bar.rfree[ch], (nit - 1) & 1, ok);
+                    if (!ok) break;
+                    if (4 * ch + 3 < t.q0 || 4 * ch >= t.q1) {
+                        mbar_arrive(&bar.rfull[ch]);  // outside the image: not read
+                        continue;
+                    }
+                    mbar_expect_tx(&bar.rfull[ch], kChunkBytes);
+                    for (int p = 0; p < 8; p++)
+                        tma_load_3d(Rs + ch * kChunkBytes + p * (kChunkBytes / 8), &q.tm, &bar.rfull[ch],
+                                    (t.x0 + 8 * p) * 4, (t.ra >> 1) + ch * (kChunkRows / 2), t.plane);
+                }
+                const float4 *src = q.ey2 + kTcPad + (t.ra >> 1);
+                for (int k = 0; k < q.nfy && ok; k++, nk++) {
+                    const int b = nk % kPhRing;
+                    if (nk >= kPhRing) wait_ok(&bar.phfree[b], ((nk / kPhRing) - 1) & 1, ok);
+                    if (!ok) break;
+                    mbar_expect_tx(&bar.phfull[b], kPhBytes);
+                    bulk_load(ph + b * kPhPairs, src + (size_t)k * q.eys2, kPhBytes, &bar.phfull[b]);
+                }
+                if (!ok) break;
+            }
+            if (!ok) atomicExch(err, GLSU_ERR_TIMEOUT);
+            // every load has landed before the CTA exits
+            for (uint32_t j = nk > kPhRing ? nk - kPhRing : 0; j < nk; j++)
+                mbar_wait_bounded(&bar.phfull[j % kPhRing], (j / kPhRing) & 1);
+            if (!ok)
+                for (int ch = 0; ch < nchunks; ch++) mbar_wait_bounded(&bar.rfull[ch], nit & 1);
+        } else if (warp == 0 || warp == 2) {
+            // ---- MMA issuers: pass 1 (warp 0) and pass 2 (warp 2) ----
+            const int W = N >> 4;                           // blocks of a window
+            const uint32_t idesc = (1u << 4) | (8u << 24);  // FP16 x FP16 -> FP32, M = 128; N / 8 goes to bit 17
+            const uint64_t bhi = umma_desc(smem_u32(tb), 128, 256), blo = umma_desc(smem_u32(tb) + N * 32, 128, 256);
+            auto issue = [&](auto pass2, uint32_t tD, uint32_t tA, uint64_t *full, uint64_t *fre, uint64_t *afull,
+                             uint64_t *afree) {
+                constexpr bool second = decltype(pass2)::value;
+                uint32_t n = 0;                 // operand slots used
+                uint32_t parity = 0, used = 0;  // per pair of blocks: parity of its next use, used before
+                for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
+                    TcTile t;
+                    const int nfy = uniform(tab.seq[tc_item<NS>(tab, nseq, item, list, listn, s, m, RW, t)].nfy);
+                    // steps from..to, outputs in blocks b0 .. b0 + nb
+                    const int from = uniform(second ? t.p0 : t.q0), to = uniform(second ? t.p1 : t.q1);
+                    const int b0 = second ? m : uniform(t.p0), nb = uniform(second ? t.nc : t.p1 - t.p0);
+                    for (int k = 0; k < nfy; k++) {
+                        int taken = 0, done = 0;  // pairs of blocks
+                        for (int st = from; st < to; st += 2, n++) {
+                            const uint32_t slot = n & 1;
+                            warp_wait(&afull[slot], (n >> 1) & 1, ok);
+#pragma unroll
+                            for (int h = 0; h < 2; h++) {
+                                if (h == 1 && st + 1 >= to) break;
+                                const int lo = max(st + h - b0, 0), hi = min(st + h + W - b0, nb);
+                                for (; 2 * taken < hi; taken++)
+                                    if ((used >> taken) & 1) warp_wait(&fre[taken], ((parity >> taken) & 1) ^ 1, ok);
+                                tc_fence_after();
+                                const uint32_t off = (uint32_t)(lo + b0 - st - h) * 32;  // 16 outputs: 512 bytes
+                                umma_step(tD + 16 * lo, tA + 32 * slot + 16 * h, bhi + off, blo + off,
+                                          idesc | ((uint32_t)(hi - lo) << 18));
+                            }
+                            umma_commit_warp(&afree[slot]);
+                            // pairs with all their products
+                            const int fin = st + 2 < to ? min(st + 2 - b0, nb) : nb;
+                            for (; 2 * done + 1 < fin || (fin == nb && 2 * done < nb); done++)
+                                umma_commit_warp(&full[done]);
+                        }
+                        const uint32_t mask = (1u << ((nb + 1) >> 1)) - 1;
+                        parity ^= mask;
+                        used |= mask;
+                    }
+                }
+            };
+            if (warp == 0) issue(std::false_type{}, tU, tA1, bar.ufull, bar.ufree, bar.a1full, bar.a1free);
+            else issue(std::true_type{}, tC, tA2, bar.cfull, bar.cfree, bar.a2full, bar.a2free);
+            if (!ok) atomicExch(err, GLSU_ERR_TIMEOUT);
+            umma_commit_warp(&bar.drain);  // every MMA has completed before TMEM is released
+            mbar_wait_bounded(&bar.drain, 0);
+        }
+    } else if (wg <= 2) {
+        // ---- A: demodulate and split 32 rows of R per slot; each warpgroup its own slot ----
+        reg_dec<Cfg::RA>();
+        const uint32_t slot = wg - 1;
+        const uint32_t a0 = tA1 + 32 * slot + lanes;
+        const unsigned char *Rw = Rs + (2 * w4) * (kChunkBytes / 8) + frow * 128;
+        uint32_t n = 0, mine = 0, nk = 0, nit = 0;  // n: slots used by both; mine: by this warpgroup
+        for (int item = blockIdx.x; item < nitems; item += gridDim.x, nit++) {
+            TcTile t;
+            const int nfy = tab.seq[tc_item<NS>(tab, nseq, item, list, listn, s, m, RW, t)].nfy;
+            for (int ch = t.q0 >> 2; ch <= (t.q1 - 1) >> 2; ch++) wait_ok(&bar.rfull[ch], nit & 1, ok);
+            for (int k = 0; k < nfy; k++, nk++) {
+                wait_ok(&bar.phfull[nk % kPhRing], (nk / kPhRing) & 1, ok);
+                const float4 *P = ph + (nk % kPhRing) * kPhPairs + frow;
+                for (int q = t.q0; q < t.q1; q += 2, n++) {
+                    if ((n & 1) != slot) continue;
+                    uint32_t o[2][8];
+                    auto half = [&](int st) {
+                        const unsigned char *base = Rw + (st >> 2) * kChunkBytes + (st & 3) * 1024;
+#pragma unroll
+                        for (int j = 0; j < 2; j++) {
+                            const float4 p = P[8 * st + 4 * j];
+                            const float2 px = make_float2(p.x, p.y), py = make_float2(p.z, p.w);
+                            const float2 ny = __fmul2_rn(py, make_float2(-1.f, -1.f));
+                            const int xo = (fcol ^ (4 * j + frow)) * 16 + 512 * j;
+#pragma unroll
+                            for (int h = 0; h < 2; h++) {
+                                const float4 x = *reinterpret_cast<const float4 *>(base + h * (kChunkBytes / 8) + xo);
+                                const float2 re = make_float2(x.x, x.y), im = make_float2(x.z, x.w);
+                                const float2 dr = __ffma2_rn(im, ny, __fmul2_rn(re, px));
+                                const float2 di = __ffma2_rn(im, px, __fmul2_rn(re, py));
+                                split2(dr, o[h][2 * j], o[h][4 + 2 * j]);
+                                split2(di, o[h][2 * j + 1], o[h][5 + 2 * j]);
+                            }
+                        }
+                    };
+                    half(q);
+                    if (mine > 0) wait_ok(&bar.a1free[slot], (mine - 1) & 1, ok);
+                    mine++;
+                    tc_fence_after();
+                    __syncwarp();
+                    tmem_st_16x128b_x4(a0, o[0]);
+                    tmem_st_16x128b_x4(a0 + (1u << 20), o[1]);
+                    if (q + 1 < t.q1) {
+                        half(q + 1);
+                        tmem_st_16x128b_x4(a0 + 16, o[0]);
+                        tmem_st_16x128b_x4(a0 + 16 + (1u << 20), o[1]);
+                    }
+                    tmem_wait_st();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&bar.a1full[slot]);
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bar.phfree[nk % kPhRing]);
+            }
+            if (lane == 0)
+                for (int ch = 0; ch < nchunks; ch++) mbar_arrive(&bar.rfree[ch]);
+        }
+        if (!ok) atomicExch(err, GLSU_ERR_TIMEOUT);
+    } else if (wg <= 4) {
+        // ---- B: threshold and split the finished rows of U, 32 per slot ----
+        reg_dec<Cfg::RT>();
+        const uint32_t slot = wg - 3;
+        const uint32_t a0 = tA2 + 32 * slot + lanes;
+        const float2 ts = make_float2(tscale, tscale);
+        uint32_t n = 0, mine = 0, parity = 0;
+        for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
+            TcTile t;
+            const TcSeq &q = tab.seq[tc_item<NS>(tab, nseq, item, list, listn, s, m, RW, t)];
+            const int nfy = q.nfy, H = q.H, urow = t.ra - s + 2 * frow, nb = t.p1 - t.p0;
+            const float thr = *q.thr * q.thr_mul * *q.kr, thr2 = thr * thr;
+            for (int k = 0; k < nfy; k++) {
+                for (int i = 0; 2 * i < nb; i++, n++) {
+                    if ((n & 1) != slot) {
+                        // not a whole phase of a barrier behind, where a wy has one pair only
+                        if (i == 0) wait_ok(&bar.ufull[0], parity & 1, ok);
+                        continue;
+                    }
+                    wait_ok(&bar.ufull[i], (parity >> i) & 1, ok);
+                    tc_fence_after();
+                    __syncwarp();
+                    uint32_t o[2][8];
+                    auto half = [&](int blk) {
+                        const uint32_t u = tU + 16 * blk + lanes;
+                        float r[2][8];
+                        tmem_ld_16x256b_x2(u, r[0]);
+                        tmem_ld_16x256b_x2(u + (1u << 20), r[1]);
+                        tmem_wait_ld();
+                        tie8(r[0]);
+                        tie8(r[1]);
+                        tmem_zero16(u);
+                        const int row = urow + 16 * (t.p0 + blk);
+#pragma unroll
+                        for (int j = 0; j < 2; j++) {
+                            const int y = row + 8 * j;  // rows outside the image carry no T
+                            const bool in0 = (unsigned)y < (unsigned)H, in1 = (unsigned)(y + 1) < (unsigned)H;
+#pragma unroll
+                            for (int h = 0; h < 2; h++) {
+                                float2 re = make_float2(r[h][4 * j], r[h][4 * j + 1]);
+                                float2 im = make_float2(r[h][4 * j + 2], r[h][4 * j + 3]);
+                                const float2 a = __ffma2_rn(im, im, __fmul2_rn(re, re));
+                                const bool k0 = in0 && a.x >= thr2, k1 = in1 && a.y >= thr2;
+                                re = make_float2(k0 ? re.x : 0.f, k1 ? re.y : 0.f);
+                                im = make_float2(k0 ? im.x : 0.f, k1 ? im.y : 0.f);
+                                split2(__fmul2_rn(re, ts), o[h][2 * j], o[h][4 + 2 * j]);
+                                split2(__fmul2_rn(im, ts), o[h][2 * j + 1], o[h][5 + 2 * j]);
+                            }
+                        }
+                    };
+                    half(2 * i);
+                    if (mine > 0) wait_ok(&bar.a2free[slot], (mine - 1) & 1, ok);
+                    mine++;
+                    tc_fence_after();
+                    __syncwarp();
+                    tmem_st_16x128b_x4(a0, o[0]);
+                    tmem_st_16x128b_x4(a0 + (1u << 20), o[1]);
+                    if (2 * i + 1 < nb) {
+                        half(2 * i + 1);
+                        tmem_st_16x128b_x4(a0 + 16, o[0]);
+                        tmem_st_16x128b_x4(a0 + 16 + (1u << 20), o[1]);
+                    }
+                    tmem_wait_st();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) {
+                        mbar_arrive(&bar.a2full[slot]);
+                        mbar_arrive(&bar.ufree[i]);
+                    }
+                }
+                parity ^= (1u << ((nb + 1) >> 1)) - 1;
+            }
+        }
+        if (!ok) atomicExch(err, GLSU_ERR_TIMEOUT);
+    } else {
+        // ---- C: modulate and sum the finished rows over wy; one block of each pair per warpgroup ----
+        reg_inc<Cfg::RC>();
+        const int par = wg - 5;
+        uint32_t nk = 0, parity = 0;
+        for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
+            TcTile t;
+            const TcSeq &q = tab.seq[tc_item<NS>(tab, nseq, item, list, listn, s, m, RW, t)];
+            const int nfy = q.nfy, poff = ((t.y0 - t.ra) >> 1) + frow;
+            float2 are[RB][2][2], aim[RB][2][2];
+#pragma unroll
+            for (int c = 0; c < RB; c++)
+#pragma unroll
+                for (int e = 0; e < 4; e++) are[c][e >> 1][e & 1] = aim[c][e >> 1][e & 1] = make_float2(0.f, 0.f);
+            for (int k = 0; k < nfy; k++, nk++) {
+                const float4 *P = ph + (nk % kPhRing) * kPhPairs + poff;
+                wait_ok(&bar.phfull[nk % kPhRing], (nk / kPhRing) & 1, ok);
+#pragma unroll
+                for (int c = 0; c < RB; c++) {
+                    if (2 * c < t.nc) {
+                        wait_ok(&bar.cfull[c], (parity >> c) & 1, ok);
+                        tc_fence_after();
+                        __syncwarp();
+                        if (2 * c + par < t.nc) {
+                            const uint32_t u = tC + 16 * (2 * c + par) + lanes;
+                            float r[2][8];
+                            tmem_ld_16x256b_x2(u, r[0]);
+                            tmem_ld_16x256b_x2(u + (1u << 20), r[1]);
+                            tmem_wait_ld();
+                            tie8(r[0]);
+                            tie8(r[1]);
+                            tmem_zero16(u);
+#pragma unroll
+                            for (int j = 0; j < 2; j++) {
+                                const float4 p = P[8 * (2 * c + par) + 4 * j];
+                                const float2 px = make_float2(p.x, p.y), py = make_float2(p.z, p.w);
+                                const float2 ny = __fmul2_rn(py, make_float2(-1.f, -1.f));
+#pragma unroll
+                                for (int h = 0; h < 2; h++) {
+                                    const float2 re = make_float2(r[h][4 * j], r[h][4 * j + 1]);
+                                    const float2 im = make_float2(r[h][4 * j + 2], r[h][4 * j + 3]);
+                                    are[c][h][j] = __ffma2_rn(px, re, __ffma2_rn(py, im, are[c][h][j]));
+                                    aim[c][h][j] = __ffma2_rn(px, im, __ffma2_rn(ny, re, aim[c][h][j]));
+                                }
+                            }
+                            tmem_wait_st();
+                        }
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&bar.cfree[c]);
+                    }
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bar.phfree[nk % kPhRing]);
+                parity ^= (1u << ((t.nc + 1) >> 1)) - 1;
+            }
+            const float mul = q.out_mul / *q.kr;
+            float2 *Cp = q.C + (size_t)t.plane * q.H * q.pitch + t.x0 + 16 * w4 + fcol;
+#pragma unroll
+            for (int c = 0; c < RB; c++)
+#pragma unroll
+                for (int j = 0; j < 2; j++) {
+                    const int y = t.y0 + 16 * (2 * c + par) + 8 * j + 2 * frow;
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        const float2 re = are[c][h][j], im = aim[c][h][j];
+                        if (y < q.H) Cp[(size_t)y * q.pitch + 8 * h] = make_float2(re.x * mul, im.x * mul);
+                        if (y + 1 < q.H) Cp[(size_t)(y + 1) * q.pitch + 8 * h] = make_float2(re.y * mul, im.y * mul);
+                    }
+                }
+        }
+        if (!ok) atomicExch(err, GLSU_ERR_TIMEOUT);
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == 0) tmem_dealloc(tmem, 512);
+}
+
+// max of |re| and |im| over the finite elements of f, as the bits of a float
+__global__ void __launch_bounds__(256) wff_absmax_kernel(const float2 *__restrict__ f, size_t n,
+                                                         uint32_t *__restrict__ out)
+{
+    float mx = 0.f;
+    for (size_t k = blockIdx.x * 256 + threadIdx.x; k < n; k += (size_t)gridDim.x * 256) {
+        const float2 v = f[k];
+        const float a = fabsf(v.x), b = fabsf(v.y);
+        if (a <= 3.402823466e38f) mx = fmaxf(mx, a);
+        if (b <= 3.402823466e38f) mx = fmaxf(mx, b);
+    }
+    const uint32_t w = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
+    if ((threadIdx.x & 31) == 0 && w) atomicMax(out, w);
+}
+
+// The power of two that R carries: with |f| <= max in each part, |R| stays below 2^15.
+__global__ void wff_tc_scale_kernel(const uint32_t *__restrict__ mx, float sum_gx, float *__restrict__ kr)
+{
+    const float b = __uint_as_float(*mx) * 1.4143f * sum_gx;
+    const int e = (int)((__float_as_uint(b) >> 23) & 255) - 126;  // b < 2^e
+    *kr = b > 0.f ? __uint_as_float((uint32_t)(127 + min(100, max(-100, 15 - e))) << 23) : 1.f;
+}
+
+// Tile heights (in pairs of blocks) whose accumulators fit the TMEM and whose
+// rows of R fit the shared memory at half-size s, largest first.
+int tc_row_blocks(int s, int *rb)
+{
+    int n = 0;
+    for (int r : {5, 4, 2})
+        if (4 * r + (s + 7) / 8 <= kBlocks && 32 * r + 16 * ((s + 3) / 4) <= kMaxChunks * kChunkRows) rb[n++] = r;
+    return n;
+}
+
+// Steps (16 image rows through one of the two passes) of one tile and wy.
+int tc_steps(int H, int s, int rw, int ty)
+{
+    const int y0 = ty * rw, y1 = std::min(H, y0 + rw);
+    const int r = std::min(H, y1 + 2 * s) - std::max(0, y0 - 2 * s), u = std::min(H, y1 + s) - std::max(0, y0 - s);
+    return (r + 31) / 16 + (u + 31) / 16;
+}
+
+// Modelled cost of a sweep of these plans with 32 rb-row tiles, in steps of
+// the busiest SM: tiles are dealt out round robin, so a few tiles more than
+// the SMs cost a whole round.
+double tc_cost(const WffPlan *const *plans, int n, int rb, int sms)
+{
+    double total = 0, items = 0, mx = 0;
+    for (int k = 0; k < n; k++) {
+        const WffPlan &P = *plans[k];
+        const int nty = (P.H + 32 * rb - 1) / (32 * rb), ncg = (P.W + kCols - 1) / kCols;
+        for (int ty = 0; ty < nty; ty++) {
+            const double st = (double)tc_steps(P.H, P.sy, 32 * rb, ty) * P.nfy;
+            total += st * ncg * P.nfx;
+            mx = std::max(mx, st);
+        }
+        items += (double)nty * ncg * P.nfx;
+    }
+    return std::ceil(items / sms) * (total / items) * 0.5 + std::max(total / sms, mx) * 0.5;
+}
+
+using Tc5 = TcCfg<5, 40, 48, 56, 128>;
+using Tc4 = TcCfg<4, 40, 56, 64, 112>;
+using Tc2 = TcCfg<2, 40, 64, 64, 88>;
+
+template <class Cfg, int NS>
+int tc_launch(const TcTable<NS> &tab, int nseq, int nitems, int grid, const WffPlan &P, const int2 *list,
+              const int *count, cudaStream_t s)
+{
+    GLSU_TRY(raise_smem_limit((const void *)wff_tc_kernel<Cfg, NS>, kSmem));
+    const int N = (2 * P.sy + 16 + 15) / 16 * 16;
+    wff_tc_kernel<Cfg, NS><<<grid, kThreads, kSmem, s>>>(tab, nseq, nitems, P.sy, (P.sy + 3) / 4, N, P.tc_tscale,
+                                                        (const uint4 *)P.d_tctaps, P.d_err, list, count);
+    GLSU_CUDA_TRY(cudaGetLastError());
+    return GLSU_OK;
+}
+
+template <int NS>
+int tc_launch_rb(int rb, const TcTable<NS> &tab, int nseq, int nitems, int grid, const WffPlan &P, const int2 *list,
+                 const int *count, cudaStream_t s)
+{
+    switch (rb) {
+    case 5: return tc_launch<Tc5, NS>(tab, nseq, nitems, grid, P, list, count, s);
+    case 4: return tc_launch<Tc4, NS>(tab, nseq, nitems, grid, P, list, count, s);
+    default: return tc_launch<Tc2, NS>(tab, nseq, nitems, grid, P, list, count, s);
+    }
+}
+
+void tc_seq(TcSeq &q, const WffPlan &P, int rw, int item0)
+{
+    q.tm = P.tmT;
+    q.ey2 = (const float4 *)P.d_ey2;
+    q.C = (float2 *)P.d_C;
+    q.thr = (const float *)P.d_thr;
+    q.kr = (const float *)P.d_kr;
+    q.H = P.H;
+    q.W = P.W;
+    q.pitch = P.pitch;
+    q.nfy = P.nfy;
+    q.eys2 = kTcPad + (P.H + 1) / 2 + kPhPairs;
+    q.ncg = (P.W + kCols - 1) / kCols;
+    q.nty = (P.H + rw - 1) / rw;
+    q.item0 = item0;
+    // U = 2^kTapShift kr N u; T = tscale U; C = 2^kTapShift sum T
+    const double taps = std::ldexp(1.0, kTapShift);
+    const double shrink = kShrink * P.sy;
+    q.thr_mul = (float)(taps / P.inv_norm * (1.0 - shrink));
+    q.out_mul = (float)(P.inv_norm / (taps * taps * (double)P.tc_tscale) * (1.0 + 2.0 * shrink));
+}
+
+}  // namespace
+
+// ---------------------------------------------------------------------------
+// host side
+// ---------------------------------------------------------------------------
+bool WffPlan::tc_supported() const { return prec == GLSU_F32 && !external_scratch && sy <= kMaxTcHalf; }
+
+// Tables of the tensor-core sweep: the B operand (K-major core matrices of 8
+// outputs x 8 inputs, hi then lo), the phasors of row pairs, the tensor map of
+// the row-pair layout of R, and the scales.
+int WffPlan::init_tc()
+{
+    if (!tc_supported()) return GLSU_OK;
+    const int N = (2 * sy + 16 + 15) / 16 * 16, eys2 = kTcPad + (H + 1) / 2 + kPhPairs;
+    std::vector<__half> tb((size_t)2 * N * 16);
+    double sum = 0, sumx = 0;
+    for (int k = 0; k <= 2 * sy; k++) sum += gy[k];
+    for (int k = 0; k <= 2 * sx; k++) sumx += gx[k];
+    for (int n = 0; n < N; n++)
+        for (int j = 0; j < 16; j++) {
+            const int k = n - j;
+            const double g = (k >= 0 && k <= 2 * sy) ? std::ldexp(gy[k], kTapShift) : 0.0;
+            const __half hi = __float2half((float)g);
+            const __half lo = __float2half((float)(g - (double)__half2float(hi)));
+            const size_t at = (size_t)(n / 8) * 128 + (size_t)(j / 8) * 64 + (n % 8) * 8 + j % 8;
+            tb[at] = hi;
+            tb[(size_t)N * 16 + at] = lo;
+        }
+    // T = tscale U stays below 2^15 as R does
+    tc_tscale = (float)std::ldexp(1.0, -(kTapShift + std::max(0, (int)std::ceil(std::log2(sum)))));
+    tc_sum_gx = (float)sumx;
+    std::vector<float> ey((size_t)nfy * eys2 * 4);
+    for (int k = 0; k < nfy; k++) {
+        const double wy = p.wyl + (double)k * p.wyi;
+        for (int i = 0; i < eys2; i++)
+            for (int r = 0; r < 2; r++) {
+                const double y = 2.0 * (i - kTcPad) + r;
+                ey[((size_t)k * eys2 + i) * 4 + r] = (float)std::cos(wy * y);
+                ey[((size_t)k * eys2 + i) * 4 + 2 + r] = (float)-std::sin(wy * y);
+            }
+    }
+    if (cudaMalloc(&d_tctaps, tb.size() * 2) != cudaSuccess || cudaMalloc(&d_ey2, ey.size() * 4) != cudaSuccess ||
+        cudaMalloc(&d_kr, 2 * sizeof(float)) != cudaSuccess)
+        return fail(GLSU_ERR_ALLOC, "cudaMalloc of the tensor-core sweep's tables failed");
+    GLSU_CUDA_TRY(cudaMemcpy(d_tctaps, tb.data(), tb.size() * 2, cudaMemcpyHostToDevice));
+    GLSU_CUDA_TRY(cudaMemcpy(d_ey2, ey.data(), ey.size() * 4, cudaMemcpyHostToDevice));
+    // scale of an input of unit modulus (DPRA); other inputs get theirs per call
+    const float kr[2] = {(float)std::ldexp(1.0, 15 - std::ilogb((float)(1.4143f * sumx)) - 1), 0.f};
+    GLSU_CUDA_TRY(cudaMemcpy(d_kr, kr, sizeof(kr), cudaMemcpyHostToDevice));
+    auto enc = get_encode_fn();
+    if (!enc) return fail(GLSU_ERR_CUDA, "cuTensorMapEncodeTiled unavailable");
+    const cuuint64_t pairs = (cuuint64_t)(H + 1) / 2;
+    cuuint64_t dims[3] = {(cuuint64_t)pitch * 4, pairs, (cuuint64_t)nfx};
+    cuuint64_t strides[2] = {(cuuint64_t)pitch * 16, pairs * pitch * 16};
+    cuuint32_t box[3] = {32, kChunkRows / 2, 1}, es[3] = {1, 1, 1};
+    if (enc(&tmT, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, d_R, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return fail(GLSU_ERR_CUDA, "cuTensorMapEncodeTiled failed");
+    return GLSU_OK;
+}
+
+void WffPlan::release_tc()
+{
+    cudaFree(d_tctaps);
+    cudaFree(d_ey2);
+    cudaFree(d_kr);
+    d_tctaps = d_ey2 = nullptr;
+    d_kr = nullptr;
+}
+
+// Scale of R for this input (d_kr[0]); d_kr[1] holds the running maximum.
+int launch_tc_scale(const WffPlan &P, const void *d_f, cudaStream_t s)
+{
+    uint32_t *mx = (uint32_t *)P.d_kr + 1;
+    GLSU_CUDA_TRY(cudaMemsetAsync(mx, 0, sizeof(uint32_t), s));
+    const size_t n = (size_t)P.W * P.H;
+    wff_absmax_kernel<<<(int)std::min<size_t>((n + 1023) / 1024, 4 * (size_t)device_sm_count()), 256, 0, s>>>(
+        (const float2 *)d_f, n, mx);
+    wff_tc_scale_kernel<<<1, 1, 0, s>>>(mx, P.tc_sum_gx, P.d_kr);
+    GLSU_CUDA_TRY(cudaGetLastError());
+    return GLSU_OK;
+}
+
+// Modelled time (ms): the steps of the busiest SM at 250 cycles each (measured
+// 247 at sigma 10 and 241 at sigma 15 on large frames), plus launch and tail.
+double tc_model_ms(const WffPlan &P)
+{
+    int rb[4];
+    const int n = tc_row_blocks(P.sy, rb);
+    const WffPlan *pp = &P;
+    double best = 1e30;
+    for (int k = 0; k < n; k++) best = std::min(best, tc_cost(&pp, 1, rb[k], 152));
+    return best * 250.0 / 1.9e6 + 0.05;
+}
+
+// The sweep of n plans of one window (half-size and sigma) as one persistent
+// launch (per 64 plans); n = 1 honours the plan's tile mask.
+int launch_tc_sweep(const WffPlan *const *plans, int n, cudaStream_t s)
+{
+    if (n <= 0) return GLSU_OK;
+    const int sms = device_sm_count();
+    int rbs[4], rb = 2;
+    const int nrb = tc_row_blocks(plans[0]->sy, rbs);
+    double best = 1e30;
+    for (int k = 0; k < nrb; k++) {
+        const double c = tc_cost(plans, n, rbs[k], sms);
+        if (c < best) {
+            best = c;
+            rb = rbs[k];
+        }
+    }
+    if (n == 1) {
+        const WffPlan &P = *plans[0];
+        TcTable<1> tab;
+        tc_seq(tab.seq[0], P, 32 * rb, 0);
+        const int tiles = tab.seq[0].ncg * tab.seq[0].nty;
+        if (!P.mask.flags) {
+            const int items = tiles * P.nfx;
+            return tc_launch_rb<1>(rb, tab, 1, items, std::min(items, sms), P, nullptr, nullptr, s);
+        }
+        // tile-masked run: the tiles whose outputs, grown by sx columns, meet a
+        // flagged tile.  A tile's results depend on its own rows of R only, and
+        // ring positions on image rows, so they are the full frame's bits.
+        if (!P.d_list) return fail(GLSU_ERR_INVALID, "tile-masked run without a tile list buffer");
+        TileMask mk = P.mask;
+        mk.my = 0;
+        mk.mx = P.sx;
+        GLSU_TRY(launch_mask_list(mk, tab.seq[0].ncg, tab.seq[0].nty, 32 * rb, kCols, P.d_list, P.d_list_count, s));
+        return tc_launch_rb<1>(rb, tab, 1, P.nfx, std::min(tiles * P.nfx, sms), P, P.d_list, P.d_list_count, s);
+    }
+    constexpr int NS = 64;
+    static thread_local TcTable<NS> tab;
+    for (int i0 = 0; i0 < n; i0 += NS) {
+        const int c = std::min(n - i0, NS);
+        int items = 0;
+        for (int k = 0; k < c; k++) {
+            const WffPlan &P = *plans[i0 + k];
+            if (P.sy != plans[0]->sy || P.p.sigma_y != plans[0]->p.sigma_y || P.mask.flags || !P.use_tc())
+                return fail(GLSU_ERR_INVALID, "batched column sweep: plans of one window only");
+            tc_seq(tab.seq[k], P, 32 * rb, items);
+            items += tab.seq[k].ncg * tab.seq[k].nty * P.nfx;
+        }
+        GLSU_TRY(tc_launch_rb<NS>(rb, tab, c, items, std::min(items, sms), *plans[i0], nullptr, nullptr, s));
+    }
+    return GLSU_OK;
+}
+
+}  // namespace glsu

@@ -53,8 +53,11 @@ extern "C" {
 
 /* Column-sweep method of the WFF2 (glsu_wff_set_method / glsu_dpra_set_method):
  * DIRECT convolves the columns with the truncated window; FFT (FP32 form
- * only) does the same in the frequency domain of each column with
- * shared-memory transforms.  AUTO (the default) picks one of the two from
+ * only) is the sweep for wide windows: banded products on the tensor cores
+ * (each FP32 value in two FP16 parts) for half-sizes round(3 sigma_y) up to
+ * 48, and beyond that, or once an FFT length or plan is set by hand, the same
+ * convolution in the frequency domain of each column with shared-memory
+ * transforms.  AUTO (the default) picks one of the two from
  * the handle's shape with a cost model of both kernels, so the choice, and
  * therefore every output bit, is the same in every process.  TIMED picks
  * the one measured fastest on this GPU (glsu_wff_tuning); its choice can
@@ -125,13 +128,15 @@ int glsu_wff_threshold(glsu_wff *h, double *thr);
  * transform plan exists (FP64 handles). */
 int glsu_wff_set_method(glsu_wff *h, int method);
 /* Column-sweep autotuner.
- * GLSU_METHOD_AUTO (the default): the FFT sweep at the shortest compiled
- * transform length >= H + 2 sy, with its default CTA width, when the cost
+ * GLSU_METHOD_AUTO (the default): GLSU_METHOD_FFT's sweep (the tensor-core
+ * sweep where it applies, else the FFT sweep at the shortest compiled
+ * transform length >= H + 2 sy with its default CTA width) when the cost
  * model puts it below 0.9 x the direct kernel's time; else the direct
  * kernel.  Decided from the shape only: deterministic.
  * GLSU_METHOD_TIMED: the handle runs the column sweep measured fastest for
  * its shape: the direct kernel, or the FFT sweep at one of the two shortest
- * compiled transform lengths, at either compiled CTA width.  The first
+ * compiled transform lengths, at either compiled CTA width, or the
+ * tensor-core sweep (reported as GLSU_METHOD_FFT).  The first
  * handle of a shape in the process times the candidates (a few launches
  * each); later handles of that shape reuse the choice.  The FFT is taken
  * only when at least 10% faster.  GLSU_AUTOTUNE=time in the environment
@@ -153,10 +158,11 @@ int glsu_wff_get_tuning(const glsu_wff *h, glsu_wff_tuning *t);
 /* Force an FFT plan variant: columns_per_cta is the length's default
  * (glsu_wff_get_tuning after glsu_wff_set_fft_length) or twice it, and
  * radix_order is 0; GLSU_ERR_UNSUPPORTED otherwise.  Takes effect when the
- * FFT sweep runs. */
+ * FFT sweep runs, which it then does in the place of the tensor-core sweep
+ * (until GLSU_METHOD_AUTO is set again). */
 int glsu_wff_set_fft_plan(glsu_wff *h, int columns_per_cta, int radix_order);
 /* Rebuild the FFT sweep's tables for another compiled transform length
- * (>= H + 2 sy) with its default CTA width. */
+ * (>= H + 2 sy) with its default CTA width, and run it as glsu_wff_set_fft_plan says. */
 int glsu_wff_set_fft_length(glsu_wff *h, int length);
 /* The compiled transform lengths >= H + 2 sy, shortest first; returns how
  * many were written (at most n; 0 without an FFT plan). */

@@ -1,0 +1,98 @@
+"""The tensor-core column sweep of the FP32 WFF2 (GLSU_METHOD_FFT without an
+FFT plan set by hand) at the sizes where its tiling can go wrong: one row and
+one column, the 16-row steps, the tile heights (64, 128, 160 rows), the 64
+columns of a tile, odd heights (rows are kept in pairs), the half-sizes at which
+the MMA width N = roundup16(2s + 16) and the tile height change, and the
+largest half-size it takes.
+
+Tolerance against the FP64 oracle, with threshold 0 so that no pixel can
+flip: per pass at most 24 truncated accumulations (2^-23 each) and the
+operands' split (2^-22), two passes, and two FP32 row filters of up to 97
+taps (2^-24 a term at worst, twice): below 2e-5 of the largest output."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+TOL = 2e-5
+
+
+def _field(shape, seed):
+    rng = np.random.default_rng(seed)
+    y, x = np.mgrid[0:shape[0], 0:shape[1]].astype(np.float64)
+    f = np.exp(1j * (0.3 * x - 0.2 * y + 0.002 * x * y)) * (1 + 0.5 * np.cos(x / 9.0))
+    return (f + 0.2 * (rng.standard_normal(shape) + 1j * rng.standard_normal(shape))).astype(np.complex64)
+
+
+def _run(glsu, f, sigy, n=3, sigx=2.0, thr=0.0, length=None):
+    import torch
+    p = glsu.WffParams(sigx, -0.4, 0.4, 0.8 / (n - 0.5), sigy, -0.4, 0.4, 0.8 / (n - 0.5), thr)
+    t = torch.from_numpy(np.ascontiguousarray(f)).cuda()
+    out = torch.full_like(t, float("nan"))
+    w = glsu.WFF2(f.shape[1], f.shape[0], "f32", p)
+    w.set_method(glsu.METHOD_FFT)
+    if length:
+        w.set_fft_length(w.tuning()["fft_length"])
+    w.run(t.data_ptr(), out.data_ptr())
+    w.close()
+    return out.cpu().numpy(), p
+
+
+SHAPES = [(1, 1), (2, 3), (15, 64), (16, 65), (17, 63), (63, 10), (64, 40), (65, 129), (159, 70), (160, 12),
+          (161, 33), (321, 66), (500, 20)]
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_tile_edges_match_oracle(glsu, oracle, shape):
+    f = _field(shape, 1)
+    for sigy in (2.0, 10.0, 16.0):
+        out, p = _run(glsu, f, sigy)
+        ref, _ = oracle.wff2(f.astype(np.complex128), *p.tuple())
+        assert np.abs(out - ref).max() <= TOL * np.abs(ref).max(), (shape, sigy)
+
+
+@pytest.mark.parametrize("half", [0, 1, 7, 8, 9, 16, 17, 24, 25, 32, 33, 40, 41, 47, 48, 49])
+def test_half_sizes_match_oracle(glsu, oracle, half):
+    f = _field((203, 70), 2)
+    out, p = _run(glsu, f, max(half, 0.1) / 3.0)
+    ref, _ = oracle.wff2(f.astype(np.complex128), *p.tuple())
+    assert np.abs(out - ref).max() <= TOL * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("e", [-60, -20, 20, 60])
+def test_scaled_input_gives_scaled_bits(glsu, e):
+    """The operands' range follows the input's, by powers of two."""
+    f = _field((90, 80), 3)
+    a, _ = _run(glsu, f, 6.0)
+    b, _ = _run(glsu, np.ldexp(f.view(np.float32), e).view(np.complex64), 6.0)
+    assert np.array_equal(np.ldexp(a.view(np.float32), e), b.view(np.float32))
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_non_finite_pixel_stays_in_its_columns(glsu, bad):
+    """Columns beyond both row filters' reach of a non-finite pixel are as
+    without it.  (The row kernels are compiled for half-sizes 12, 20, ... and
+    multiply by zero taps up to that: their reach, here 12, is the compiled one.)"""
+    f = _field((120, 200), 4)
+    f[50, 30] = 0
+    a, _ = _run(glsu, f, 5.0, sigx=4.0)
+    f[50, 30] = bad
+    b, _ = _run(glsu, f, 5.0, sigx=4.0)
+    far = 30 + 2 * 12 + 1
+    assert np.array_equal(a[:, far:], b[:, far:])
+
+
+def test_zero_field_and_high_threshold(glsu):
+    f = _field((70, 90), 5)
+    for g, thr in ((np.zeros_like(f), 0.0), (f, 1e30)):
+        out, _ = _run(glsu, g, 8.0, thr=thr)
+        assert np.array_equal(out, np.zeros_like(out))
+
+
+def test_fft_length_by_hand_runs_the_fft_sweep(glsu):
+    """Setting a length selects the FFT kernels, whose bits differ; both agree to the tolerance."""
+    f = _field((300, 130), 6)
+    a, _ = _run(glsu, f, 10.0, n=5)
+    b, _ = _run(glsu, f, 10.0, n=5, length=True)
+    assert not np.array_equal(a, b)
+    assert np.abs(a - b).max() <= TOL * np.abs(b).max()
