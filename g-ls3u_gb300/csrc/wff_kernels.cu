@@ -83,7 +83,7 @@ template <typename T, int S, bool PACK>
 __global__ void __launch_bounds__(256) wff_rows_demod_kernel(const C2<T> *__restrict__ f, int W, int H,
                                                              int pitch, const C2<T> *__restrict__ ex, int nfx,
                                                              C2<T> *__restrict__ R, Taps<T, S> gx, TileMask tm,
-                                                             const T *__restrict__ kr)
+                                                             const T *__restrict__ kr, int zplanes)
 {
     using G = RowGeom<T, S>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -105,7 +105,8 @@ __global__ void __launch_bounds__(256) wff_rows_demod_kernel(const C2<T> *__rest
     const size_t exs = (size_t)pitch + 2 * kPhasorPad;
     const size_t plane = (size_t)H * pitch;
     const C2<T> *row = ft + lane * G::IN_STRIDE + w * kRowK;
-    for (int i = 0; i < nfx; i++) {
+    const int i1 = min(nfx, (int)(blockIdx.z + 1) * zplanes);
+    for (int i = blockIdx.z * zplanes; i < i1; i++) {
         const C2<T> *exi = ex + i * exs + kPhasorPad + (x0 - S + w * kRowK);
         T ar[kRowK], ai[kRowK];
 #pragma unroll
@@ -374,6 +375,26 @@ template <> __device__ __forceinline__ double wrap_atan2<double>(double a)
     return atan2(s, c);
 }
 
+// One pixel of the filtered field: stored (MODE 0), or the DPRA update
+// (DPRA/dpra_hybrid.cu:297-315, DPRA/dpra_cpu.cpp:243-249).  MODE 2 leaves the
+// wrapped change t for the spatial unwrapping, which adds dphi_ref afterwards
+// (MatLab/fp_ls3u.m:104).
+template <typename T, int MODE>
+__device__ __forceinline__ void final_pixel(C2<T> v, size_t id, C2<T> *__restrict__ out, const T *__restrict__ phiref,
+                                            const T *__restrict__ dphiref, T *__restrict__ phicurr,
+                                            T *__restrict__ dphi)
+{
+    if (MODE == 0) {
+        out[id] = v;
+    } else {
+        const T t = atan2(v.y, v.x);
+        const T pr = phiref[id];
+        phicurr[id] = wrap_atan2<T>(t + pr);
+        dphi[id] = (MODE == 1) ? dphiref[id] + t : t;
+    }
+}
+
+// MODE 3: this CTA's planes only, into partial sum blockIdx.z of out.
 template <typename T, int S, int MODE>
 __global__ void __launch_bounds__(256) wff_rows_final_kernel(const C2<T> *__restrict__ Cin, int W, int H,
                                                              int pitch, const C2<T> *__restrict__ ex, int nfx,
@@ -381,7 +402,7 @@ __global__ void __launch_bounds__(256) wff_rows_final_kernel(const C2<T> *__rest
                                                              const T *__restrict__ phiref,
                                                              const T *__restrict__ dphiref,
                                                              T *__restrict__ phicurr, T *__restrict__ dphi,
-                                                             TileMask tm)
+                                                             TileMask tm, int zplanes)
 {
     using G = RowGeom<T, S>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -400,7 +421,8 @@ __global__ void __launch_bounds__(256) wff_rows_final_kernel(const C2<T> *__rest
         oii[k] = 0;
     }
     const C2<T> *row = ft + lane * G::IN_STRIDE + w * kRowK;
-    for (int i = 0; i < nfx; i++) {
+    const int i1 = min(nfx, (int)(blockIdx.z + 1) * zplanes);
+    for (int i = blockIdx.z * zplanes; i < i1; i++) {
         const C2<T> *Ci = Cin + i * plane;
         for (int e = tid; e < kRowTileRows * G::IN_W; e += 256) {
             const int r = e / G::IN_W, c = e - r * G::IN_W;
@@ -448,18 +470,29 @@ __global__ void __launch_bounds__(256) wff_rows_final_kernel(const C2<T> *__rest
         if (tm.flags && !tm.at(gy, gxx)) continue;
         const size_t id = (size_t)gy * W + gxx;
         const C2<T> v = ot[r * G::OUT_STRIDE + c];
-        if (MODE == 0) {
-            out[id] = v;
-        } else {
-            // DPRA update (DPRA/dpra_hybrid.cu:297-315, DPRA/dpra_cpu.cpp:243-249)
-            const T t = atan2(v.y, v.x);
-            const T pr = phiref[id];
-            phicurr[id] = wrap_atan2<T>(t + pr);
-            // MODE 2 leaves the wrapped change t for the spatial unwrapping,
-            // which adds dphi_ref afterwards (MatLab/fp_ls3u.m:104)
-            dphi[id] = (MODE == 1) ? dphiref[id] + t : t;
-        }
+        if (MODE == 3) out[(size_t)blockIdx.z * W * H + id] = v;
+        else final_pixel<T, MODE>(v, id, out, phiref, dphiref, phicurr, dphi);
     }
+}
+
+// Sum of the nz partial sums of the final row pass, in plane order, and what
+// MODE does with it.
+template <typename T, int MODE>
+__global__ void __launch_bounds__(256) wff_rows_sum_kernel(const C2<T> *__restrict__ part, int nz, int W, int H,
+                                                           C2<T> *__restrict__ out, const T *__restrict__ phiref,
+                                                           const T *__restrict__ dphiref, T *__restrict__ phicurr,
+                                                           T *__restrict__ dphi, TileMask tm)
+{
+    const int x = blockIdx.x * 32 + (threadIdx.x & 31), y = blockIdx.y * 8 + (threadIdx.x >> 5);
+    if (x >= W || y >= H || (tm.flags && !tm.at(y, x))) return;
+    const size_t n = (size_t)W * H, id = (size_t)y * W + x;
+    C2<T> v = part[id];
+    for (int z = 1; z < nz; z++) {
+        const C2<T> p = part[z * n + id];
+        v.x += p.x;
+        v.y += p.y;
+    }
+    final_pixel<T, MODE>(v, id, out, phiref, dphiref, phicurr, dphi);
 }
 
 // ---------------------------------------------------------------------------
@@ -727,15 +760,29 @@ static TileMask with_margins(TileMask m, int my, int mx)
     return m;
 }
 
+// Planes per CTA of the row passes.  A frame has (pitch/128) x (H/32) row
+// tiles, 16 at 256 x 256: below one wave (two CTAs per SM) the planes are
+// dealt out over blockIdx.z to fill it.  Both row passes of a 256 x 256 frame
+// with sigma 20 and 7 x 7 frequencies: 164 -> 60 us; the 480 x 640, sigma 10
+// frame 721 -> 593 us in all.  At 1024^2 (256 tiles) four CTAs per SM
+// instead of the unsplit pass made the frame 30 us slower.
+static int rows_zplanes(const WffPlan &P)
+{
+    const int tiles = (P.pitch / kRowTileCols) * ((P.H + kRowTileRows - 1) / kRowTileRows);
+    const int z = std::max(1, std::min(P.nfx, 2 * 152 / tiles));
+    return (P.nfx + z - 1) / z;
+}
+
 template <typename T, int S, bool PACK>
 static int launch_rows_demod_t(const WffPlan &P, const void *d_f, cudaStream_t s)
 {
     using G = RowGeom<T, S>;
     GLSU_TRY(raise_smem_limit((const void *)wff_rows_demod_kernel<T, S, PACK>, (int)G::SMEM));
-    dim3 grid(P.pitch / kRowTileCols, (P.H + kRowTileRows - 1) / kRowTileRows);
+    const int zp = rows_zplanes(P);
+    dim3 grid(P.pitch / kRowTileCols, (P.H + kRowTileRows - 1) / kRowTileRows, (P.nfx + zp - 1) / zp);
     wff_rows_demod_kernel<T, S, PACK><<<grid, 256, G::SMEM, s>>>(
         (const C2<T> *)d_f, P.W, P.H, P.pitch, (const C2<T> *)P.d_ex, P.nfx, (C2<T> *)P.d_R,
-        make_taps<T, S>(P.gx, P.sx, 1.0), with_margins(P.mask, 2 * P.sy, P.sx), (const T *)P.d_kr);
+        make_taps<T, S>(P.gx, P.sx, 1.0), with_margins(P.mask, 2 * P.sy, P.sx), (const T *)P.d_kr, zp);
     GLSU_CUDA_TRY(cudaGetLastError());
     return GLSU_OK;
 }
@@ -793,16 +840,34 @@ template <typename T, int S> static int launch_cols(const WffPlan &P, cudaStream
 }
 
 template <typename T, int S, int MODE>
-static int launch_final(const WffPlan &P, void *d_out, const void *phiref, const void *dphiref, void *phicurr,
-                        void *dphi, cudaStream_t s)
+static int launch_final_t(const WffPlan &P, void *d_out, const void *phiref, const void *dphiref, void *phicurr,
+                          void *dphi, int zp, cudaStream_t s)
 {
     using G = RowGeom<T, S>;
     GLSU_TRY(raise_smem_limit((const void *)wff_rows_final_kernel<T, S, MODE>, (int)G::SMEM));
-    dim3 grid(P.pitch / kRowTileCols, (P.H + kRowTileRows - 1) / kRowTileRows);
+    dim3 grid(P.pitch / kRowTileCols, (P.H + kRowTileRows - 1) / kRowTileRows, (P.nfx + zp - 1) / zp);
     wff_rows_final_kernel<T, S, MODE><<<grid, 256, G::SMEM, s>>>(
         (const C2<T> *)P.d_C, P.W, P.H, P.pitch, (const C2<T> *)P.d_ex, P.nfx,
         make_taps<T, S>(P.gx, P.sx, P.scale * P.inv_norm), (C2<T> *)d_out, (const T *)phiref, (const T *)dphiref,
-        (T *)phicurr, (T *)dphi, with_margins(P.mask, 0, 0));
+        (T *)phicurr, (T *)dphi, with_margins(P.mask, 0, 0), zp);
+    GLSU_CUDA_TRY(cudaGetLastError());
+    return GLSU_OK;
+}
+
+// The planes split as in the first row pass: each CTA's partial sums go to
+// the R planes, which the column sweep is done with, and one more kernel adds
+// them.  The split follows the shape alone, so a tile-masked run gives the
+// full frame's bits.
+template <typename T, int S, int MODE>
+static int launch_final(const WffPlan &P, void *d_out, const void *phiref, const void *dphiref, void *phicurr,
+                        void *dphi, cudaStream_t s)
+{
+    const int zp = rows_zplanes(P), nz = (P.nfx + zp - 1) / zp;
+    if (nz == 1) return launch_final_t<T, S, MODE>(P, d_out, phiref, dphiref, phicurr, dphi, zp, s);
+    GLSU_TRY((launch_final_t<T, S, 3>(P, P.d_R, nullptr, nullptr, nullptr, nullptr, zp, s)));
+    wff_rows_sum_kernel<T, MODE><<<dim3((P.W + 31) / 32, (P.H + 7) / 8), 256, 0, s>>>(
+        (const C2<T> *)P.d_R, nz, P.W, P.H, (C2<T> *)d_out, (const T *)phiref, (const T *)dphiref, (T *)phicurr,
+        (T *)dphi, with_margins(P.mask, 0, 0));
     GLSU_CUDA_TRY(cudaGetLastError());
     return GLSU_OK;
 }
