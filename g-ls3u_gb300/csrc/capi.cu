@@ -483,6 +483,10 @@ static void get_tuning(const WffPlan &P, glsu_wff_tuning *t)
     t->fft_length = P.fft_L;
     t->fft_columns = P.fft_nc;
     t->fft_radix_order = P.fft_order;
+    if (P.use_fft64()) {
+        t->method = GLSU_METHOD_FFT;
+        t->fft_length = P.fft64_L;
+    }
     t->tuned = P.tuned ? (P.timed ? 1 : 2) : 0;
     t->ms_direct = P.tune_ms_direct;
     t->ms_fft = P.tune_ms_fft;

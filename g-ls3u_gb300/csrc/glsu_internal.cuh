@@ -191,6 +191,13 @@ struct WffPlan {
     // where it does not fit (the plan is then unchanged).
     int set_fft_plan(int nc, int order);
 
+    // FFT column sweep of FP64 handles (wff_colfft64.cu), under AUTO.
+    int fft64_L = 0;
+    void *d_h64 = nullptr;   // nfy x fft64_L real spectra of the modulated windows
+    void *d_tw64 = nullptr;  // fft64_L twiddles
+    int init_colfft64();
+    bool use_fft64() const { return fft64_L > 0 && d_h64 && d_tw64 && column_method() == GLSU_METHOD_FFT; }
+
     // Autotuner (wff_colfft.cu): with GLSU_METHOD_AUTO the column sweep is
     // chosen from the shape by a cost model (deterministic); with
     // GLSU_METHOD_TIMED it is the candidate (direct kernel or FFT plan
@@ -234,6 +241,7 @@ int fft_length_candidates(const WffPlan &P, int *out, int n);
 int launch_column_sweep(WffPlan &P, cudaStream_t s);
 
 int launch_colfft(const WffPlan &P, cudaStream_t s);
+int launch_colfft64(const WffPlan &P, cudaStream_t s);
 // The FFT column sweep of n plans of one transform length (each running the
 // FFT sweep, no tile mask) as one persistent launch over their work list.
 int launch_colfft_batch(const WffPlan *const *plans, int n, cudaStream_t s);

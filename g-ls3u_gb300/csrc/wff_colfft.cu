@@ -62,7 +62,7 @@ static bool ncol_ok(int L, int nc, int pitch)
 
 int WffPlan::init_colfft()
 {
-    if (prec != GLSU_F32) return GLSU_OK;
+    if (prec != GLSU_F32) return init_colfft64();
     int L;
     if (length_candidates(H + 2 * sy, &L, 1) < 1) return GLSU_OK;  // taller than the longest plan: direct kernel
     return set_fft_len(L);
@@ -149,7 +149,10 @@ void WffPlan::release_colfft()
 {
     cudaFree(d_khat);
     cudaFree(d_tw);
-    d_khat = d_tw = nullptr;
+    cudaFree(d_h64);
+    cudaFree(d_tw64);
+    d_khat = d_tw = d_h64 = d_tw64 = nullptr;
+    fft64_L = 0;
     fft_L = 0;
 }
 
@@ -311,9 +314,10 @@ int WffPlan::autotune(cudaStream_t s)
     timed = false;
     auto_method = GLSU_METHOD_DIRECT;
     tune_ms_direct = tune_ms_fft = 0;
-    if (prec != GLSU_F32 || fft_L == 0) return GLSU_OK;
     const char *env = std::getenv("GLSU_AUTOTUNE");
     if (env && env[0] == '0') return GLSU_OK;
+    if (fft64_L > 0) auto_method = GLSU_METHOD_FFT;
+    if (prec != GLSU_F32 || fft_L == 0) return GLSU_OK;
     const bool want_timing = method == GLSU_METHOD_TIMED || (env && std::strcmp(env, "time") == 0);
     if (!want_timing) return choose_by_model();
     timed = true;

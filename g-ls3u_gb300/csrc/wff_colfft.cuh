@@ -35,46 +35,59 @@
 namespace glsu {
 namespace colfft {
 
-__device__ __forceinline__ float2 cmul(float2 a, float2 b)
+// V: float2 or double2
+template <typename V> struct RealOf;
+template <> struct RealOf<float2> { using T = float; };
+template <> struct RealOf<double2> { using T = double; };
+template <typename V> using Real = typename RealOf<V>::T;
+template <typename V> __device__ __forceinline__ V mkv(Real<V> x, Real<V> y)
 {
-    return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+    V v;
+    v.x = x;
+    v.y = y;
+    return v;
 }
-__device__ __forceinline__ float2 conjf2(float2 a) { return make_float2(a.x, -a.y); }
-__device__ __forceinline__ float2 mul_mi(float2 a) { return make_float2(a.y, -a.x); }  // a * (-i)
+
+template <typename V> __device__ __forceinline__ V cmul(V a, V b)
+{
+    return mkv<V>(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+}
+template <typename V> __device__ __forceinline__ V conjf2(V a) { return mkv<V>(a.x, -a.y); }
+template <typename V> __device__ __forceinline__ V mul_mi(V a) { return mkv<V>(a.y, -a.x); }  // a * (-i)
 
 // forward DFTs of 2, 3, 4, 5 and 8 points in registers (exponent -2 pi i / R)
-__device__ __forceinline__ void dft2(float2 *v)
+template <typename V> __device__ __forceinline__ void dft2(V *v)
 {
-    const float2 a = v[0], b = v[1];
-    v[0] = make_float2(a.x + b.x, a.y + b.y);
-    v[1] = make_float2(a.x - b.x, a.y - b.y);
+    const V a = v[0], b = v[1];
+    v[0] = mkv<V>(a.x + b.x, a.y + b.y);
+    v[1] = mkv<V>(a.x - b.x, a.y - b.y);
 }
 
-__device__ __forceinline__ void dft4(float2 *v)
+template <typename V> __device__ __forceinline__ void dft4(V *v)
 {
-    const float2 a0 = make_float2(v[0].x + v[2].x, v[0].y + v[2].y);
-    const float2 a1 = make_float2(v[0].x - v[2].x, v[0].y - v[2].y);
-    const float2 a2 = make_float2(v[1].x + v[3].x, v[1].y + v[3].y);
-    const float2 a3 = mul_mi(make_float2(v[1].x - v[3].x, v[1].y - v[3].y));
-    v[0] = make_float2(a0.x + a2.x, a0.y + a2.y);
-    v[2] = make_float2(a0.x - a2.x, a0.y - a2.y);
-    v[1] = make_float2(a1.x + a3.x, a1.y + a3.y);
-    v[3] = make_float2(a1.x - a3.x, a1.y - a3.y);
+    const V a0 = mkv<V>(v[0].x + v[2].x, v[0].y + v[2].y);
+    const V a1 = mkv<V>(v[0].x - v[2].x, v[0].y - v[2].y);
+    const V a2 = mkv<V>(v[1].x + v[3].x, v[1].y + v[3].y);
+    const V a3 = mul_mi(mkv<V>(v[1].x - v[3].x, v[1].y - v[3].y));
+    v[0] = mkv<V>(a0.x + a2.x, a0.y + a2.y);
+    v[2] = mkv<V>(a0.x - a2.x, a0.y - a2.y);
+    v[1] = mkv<V>(a1.x + a3.x, a1.y + a3.y);
+    v[3] = mkv<V>(a1.x - a3.x, a1.y - a3.y);
 }
 
-__device__ __forceinline__ void dft8(float2 *v)
+template <typename V> __device__ __forceinline__ void dft8(V *v)
 {
     // X[2q] = DFT4(v_r + v_{r+4}), X[2q+1] = DFT4((v_r - v_{r+4}) w8^r), w8 = e^{-i pi/4}
-    const float h = 0.70710678118654752f;
-    float2 b[4], c[4];
+    const Real<V> h = (Real<V>)0.70710678118654752440;
+    V b[4], c[4];
 #pragma unroll
     for (int r = 0; r < 4; r++) {
-        b[r] = make_float2(v[r].x + v[r + 4].x, v[r].y + v[r + 4].y);
-        c[r] = make_float2(v[r].x - v[r + 4].x, v[r].y - v[r + 4].y);
+        b[r] = mkv<V>(v[r].x + v[r + 4].x, v[r].y + v[r + 4].y);
+        c[r] = mkv<V>(v[r].x - v[r + 4].x, v[r].y - v[r + 4].y);
     }
-    c[1] = make_float2(h * (c[1].x + c[1].y), h * (c[1].y - c[1].x));
+    c[1] = mkv<V>(h * (c[1].x + c[1].y), h * (c[1].y - c[1].x));
     c[2] = mul_mi(c[2]);
-    c[3] = make_float2(h * (c[3].y - c[3].x), -h * (c[3].x + c[3].y));
+    c[3] = mkv<V>(h * (c[3].y - c[3].x), -h * (c[3].x + c[3].y));
     dft4(b);
     dft4(c);
 #pragma unroll
@@ -84,40 +97,40 @@ __device__ __forceinline__ void dft8(float2 *v)
     }
 }
 
-__device__ __forceinline__ void dft3(float2 *v)
+template <typename V> __device__ __forceinline__ void dft3(V *v)
 {
-    const float s3 = 0.86602540378443865f;  // sin(2 pi / 3)
-    const float2 t1 = make_float2(v[1].x + v[2].x, v[1].y + v[2].y);
-    const float2 t2 = make_float2(v[1].x - v[2].x, v[1].y - v[2].y);
-    const float2 m = make_float2(v[0].x - 0.5f * t1.x, v[0].y - 0.5f * t1.y);
-    const float2 j = make_float2(s3 * t2.y, -s3 * t2.x);  // -i s3 t2
-    v[0] = make_float2(v[0].x + t1.x, v[0].y + t1.y);
-    v[1] = make_float2(m.x + j.x, m.y + j.y);
-    v[2] = make_float2(m.x - j.x, m.y - j.y);
+    const Real<V> s3 = (Real<V>)0.86602540378443864676;  // sin(2 pi / 3)
+    const V t1 = mkv<V>(v[1].x + v[2].x, v[1].y + v[2].y);
+    const V t2 = mkv<V>(v[1].x - v[2].x, v[1].y - v[2].y);
+    const V m = mkv<V>(v[0].x - (Real<V>)0.5 * t1.x, v[0].y - (Real<V>)0.5 * t1.y);
+    const V j = mkv<V>(s3 * t2.y, -s3 * t2.x);  // -i s3 t2
+    v[0] = mkv<V>(v[0].x + t1.x, v[0].y + t1.y);
+    v[1] = mkv<V>(m.x + j.x, m.y + j.y);
+    v[2] = mkv<V>(m.x - j.x, m.y - j.y);
 }
 
-__device__ __forceinline__ void dft5(float2 *v)
+template <typename V> __device__ __forceinline__ void dft5(V *v)
 {
-    const float c1 = 0.30901699437494742f, c2 = -0.80901699437494742f;  // cos(2pi/5), cos(4pi/5)
-    const float s1 = 0.95105651629515357f, s2 = 0.58778525229247313f;   // sin(2pi/5), sin(4pi/5)
-    const float2 a1 = make_float2(v[1].x + v[4].x, v[1].y + v[4].y);
-    const float2 b1 = make_float2(v[1].x - v[4].x, v[1].y - v[4].y);
-    const float2 a2 = make_float2(v[2].x + v[3].x, v[2].y + v[3].y);
-    const float2 b2 = make_float2(v[2].x - v[3].x, v[2].y - v[3].y);
-    const float2 m1 = make_float2(v[0].x + c1 * a1.x + c2 * a2.x, v[0].y + c1 * a1.y + c2 * a2.y);
-    const float2 m2 = make_float2(v[0].x + c2 * a1.x + c1 * a2.x, v[0].y + c2 * a1.y + c1 * a2.y);
-    const float2 n1 = make_float2(s1 * b1.x + s2 * b2.x, s1 * b1.y + s2 * b2.y);
-    const float2 n2 = make_float2(s2 * b1.x - s1 * b2.x, s2 * b1.y - s1 * b2.y);
-    const float2 j1 = make_float2(n1.y, -n1.x);  // -i n1
-    const float2 j2 = make_float2(n2.y, -n2.x);
-    v[0] = make_float2(v[0].x + a1.x + a2.x, v[0].y + a1.y + a2.y);
-    v[1] = make_float2(m1.x + j1.x, m1.y + j1.y);
-    v[4] = make_float2(m1.x - j1.x, m1.y - j1.y);
-    v[2] = make_float2(m2.x + j2.x, m2.y + j2.y);
-    v[3] = make_float2(m2.x - j2.x, m2.y - j2.y);
+    const Real<V> c1 = (Real<V>)0.30901699437494742410, c2 = (Real<V>)-0.80901699437494742410;  // cos(2pi/5), cos(4pi/5)
+    const Real<V> s1 = (Real<V>)0.95105651629515357212, s2 = (Real<V>)0.58778525229247312917;   // sin(2pi/5), sin(4pi/5)
+    const V a1 = mkv<V>(v[1].x + v[4].x, v[1].y + v[4].y);
+    const V b1 = mkv<V>(v[1].x - v[4].x, v[1].y - v[4].y);
+    const V a2 = mkv<V>(v[2].x + v[3].x, v[2].y + v[3].y);
+    const V b2 = mkv<V>(v[2].x - v[3].x, v[2].y - v[3].y);
+    const V m1 = mkv<V>(v[0].x + c1 * a1.x + c2 * a2.x, v[0].y + c1 * a1.y + c2 * a2.y);
+    const V m2 = mkv<V>(v[0].x + c2 * a1.x + c1 * a2.x, v[0].y + c2 * a1.y + c1 * a2.y);
+    const V n1 = mkv<V>(s1 * b1.x + s2 * b2.x, s1 * b1.y + s2 * b2.y);
+    const V n2 = mkv<V>(s2 * b1.x - s1 * b2.x, s2 * b1.y - s1 * b2.y);
+    const V j1 = mkv<V>(n1.y, -n1.x);  // -i n1
+    const V j2 = mkv<V>(n2.y, -n2.x);
+    v[0] = mkv<V>(v[0].x + a1.x + a2.x, v[0].y + a1.y + a2.y);
+    v[1] = mkv<V>(m1.x + j1.x, m1.y + j1.y);
+    v[4] = mkv<V>(m1.x - j1.x, m1.y - j1.y);
+    v[2] = mkv<V>(m2.x + j2.x, m2.y + j2.y);
+    v[3] = mkv<V>(m2.x - j2.x, m2.y - j2.y);
 }
 
-template <int R> __device__ __forceinline__ void dft(float2 *v)
+template <int R, typename V> __device__ __forceinline__ void dft(V *v)
 {
     if constexpr (R == 2) dft2(v);
     else if constexpr (R == 4) dft4(v);
@@ -172,9 +185,8 @@ template <int T> __device__ __forceinline__ void col_sync(int col)
 // the registers in cyclic order (v[m] = x[t + T m]); else pass p-1's
 // exchange buffer.  Output: pass p's exchange buffer, or for the last pass
 // the registers in cyclic order.  tw[e] = e^{-2 pi i e / L}.
-template <class P, int p>
-__device__ __forceinline__ void pass(float2 (&v)[P::Q], float2 *__restrict__ xb, const float2 *__restrict__ tw, int t,
-                                     int col)
+template <class P, int p, typename V>
+__device__ __forceinline__ void pass(V (&v)[P::Q], V *__restrict__ xb, const V *__restrict__ tw, int t, int col)
 {
     constexpr int L = P::L, T = P::T, Q = P::Q, R = P::radix(p), NB = Q / R, Ns = P::ns(p);
     constexpr bool first = p == 0, last = p == P::NP - 1;
@@ -192,10 +204,10 @@ __device__ __forceinline__ void pass(float2 (&v)[P::Q], float2 *__restrict__ xb,
             }
         col_sync<T>(col);  // every read of the buffer done before this pass writes it
     }
-    float2 o[last ? Q : 1];
+    V o[last ? Q : 1];
 #pragma unroll
     for (int q = 0; q < NB; q++) {
-        float2 a[R];
+        V a[R];
 #pragma unroll
         for (int r = 0; r < R; r++) a[r] = first ? v[q + r * NB] : v[q * R + r];
         if constexpr (Ns > 1) {
@@ -222,9 +234,8 @@ __device__ __forceinline__ void pass(float2 (&v)[P::Q], float2 *__restrict__ xb,
     }
 }
 
-template <class P>
-__device__ __forceinline__ void fft(float2 (&v)[P::Q], float2 *__restrict__ xb, const float2 *__restrict__ tw, int t,
-                                    int col)
+template <class P, typename V>
+__device__ __forceinline__ void fft(V (&v)[P::Q], V *__restrict__ xb, const V *__restrict__ tw, int t, int col)
 {
     pass<P, 0>(v, xb, tw, t, col);
     pass<P, 1>(v, xb, tw, t, col);

@@ -879,6 +879,7 @@ template <typename T> static int launch_cols_any(WffPlan &P, cudaStream_t s)
         return launch_tc_sweep(&one, 1, s);
     }
     if (sizeof(T) == 4 && P.use_colfft()) return launch_colfft(P, s);
+    if (sizeof(T) == 8 && P.use_fft64() && !P.mask.flags) return launch_colfft64(P, s);
     switch (P.syi) {
     case 12: return launch_cols<T, 12>(P, s);
     case 20: return launch_cols<T, 20>(P, s);
