@@ -1525,7 +1525,8 @@ extern "C" int glsu_aia_create(glsu_aia **out, int M, int cols, int rows)
                   cudaMalloc((void **)&h->d_phi, sizeof(float) * h->N) == cudaSuccess &&
                   cudaMalloc((void **)&h->dev.d_part, sizeof(double) * nv * h->dev.nblocks) == cudaSuccess &&
                   cudaMalloc((void **)&h->dev.d_state, sizeof(double) * (2 * M + 3)) == cudaSuccess &&
-                  cudaMalloc((void **)&h->dev.d_done, sizeof(int)) == cudaSuccess;
+                  cudaMalloc((void **)&h->dev.d_done, sizeof(int)) == cudaSuccess &&
+                  cudaMalloc(&h->dev.d_tab, aia_tables_bytes()) == cudaSuccess;
         if (!ok) rc = fail(GLSU_ERR_ALLOC, "AIA buffer allocation failed");
     }
     if (rc == GLSU_OK && (cudaEventCreate(&h->t0) != cudaSuccess || cudaEventCreate(&h->t1) != cudaSuccess))
@@ -1547,6 +1548,7 @@ extern "C" int glsu_aia_destroy(glsu_aia *h)
     cudaFree(h->dev.d_part);
     cudaFree(h->dev.d_state);
     cudaFree(h->dev.d_done);
+    cudaFree(h->dev.d_tab);
     if (h->t0) cudaEventDestroy(h->t0);
     if (h->t1) cudaEventDestroy(h->t1);
     if (h->own_stream && h->stream) cudaStreamDestroy(h->stream);
@@ -1579,13 +1581,10 @@ static int aia_core(glsu_aia *h, const void *d_frames, int img_type, float *d_ph
     cudaStream_t s = h->stream;
     GLSU_CUDA_TRY(cudaEventRecord(h->t0, s));
     GLSU_TRY(aia_launch_init(h->dev, dd.data(), s));
-    for (int it = 0; it < max_iter; it++) {
-        GLSU_TRY(aia_launch_pass(h->dev, img_type, d_frames, 0, nullptr, s));
-        GLSU_TRY(aia_launch_solve(h->dev, max_iter, (double)max_err, s));
-    }
+    for (int it = 0; it < max_iter; it++)
+        GLSU_TRY(aia_launch_iteration(h->dev, img_type, d_frames, max_iter, (double)max_err, s));
     GLSU_CUDA_TRY(cudaEventRecord(h->t1, s));
-    GLSU_TRY(aia_launch_pass(h->dev, img_type, d_frames, 1, d_phi, s));
-    GLSU_TRY(aia_launch_finalize(h->dev, d_phi, s));
+    GLSU_TRY(aia_launch_finalize(h->dev, img_type, d_frames, d_phi, s));
     std::vector<double> st(2 * h->M + 3);
     GLSU_CUDA_TRY(cudaMemcpyAsync(st.data(), h->dev.d_state, sizeof(double) * st.size(), cudaMemcpyDeviceToHost, s));
     GLSU_CUDA_TRY(cudaStreamSynchronize(s));

@@ -320,12 +320,13 @@ struct AiaDev {
     double *d_part = nullptr;   // nblocks x (5 + 3M) partial sums
     double *d_state = nullptr;  // deltas, old deltas, err, iteration, flags
     int *d_done = nullptr;
+    void *d_tab = nullptr;  // aia_tables_bytes(): the phi-step's tables and the launch's ticket
     int err_mode = GLSU_AIA_ERR_ABS;  // convergence measure (glsu_aia_set_convergence)
 };
-int aia_launch_pass(const AiaDev &a, int img_type, const void *d_frames, int final_pass, float *d_phi,
-                    cudaStream_t s);
-int aia_launch_solve(const AiaDev &a, int max_iter, double max_err, cudaStream_t s);
+size_t aia_tables_bytes();
 int aia_launch_init(const AiaDev &a, const double *h_deltas, cudaStream_t s);
-int aia_launch_finalize(const AiaDev &a, float *d_phi, cudaStream_t s);
+int aia_launch_iteration(const AiaDev &a, int img_type, const void *d_frames, int max_iter, double max_err,
+                         cudaStream_t s);
+int aia_launch_finalize(const AiaDev &a, int img_type, const void *d_frames, float *d_phi, cudaStream_t s);
 
 }  // namespace glsu
