@@ -13,7 +13,6 @@
 namespace glsu {
 
 constexpr int kSurPixBlocks = 152 * 8;  // grid of the per-pixel CUDA-core kernels
-constexpr int kSurDbPix = 4096;         // pixels per block of the bias-gradient sums
 
 static int grid_for(size_t n) { return (int)std::min<size_t>((n + 255) / 256, kSurPixBlocks); }
 
@@ -66,10 +65,7 @@ int SurNet::init(int batch, int width, int height, const int *dilations, bool tr
              A((void **)&d_y, n * 8) &&
              A((void **)&d_loss, 8);
         nbs = sur_dw_small_blocks(B, H, W);
-        ndb = (int)((n + kSurDbPix - 1) / kSurDbPix);
-        const size_t part = std::max<size_t>(std::max<size_t>((size_t)device_sm_count() * 9216,
-                                                              (size_t)nbs * kSurL0Params),
-                                             (size_t)ndb * 32);
+        const size_t part = std::max<size_t>((size_t)device_sm_count() * kWgCols, (size_t)nbs * kSurL0Params);
         ok = ok && A((void **)&d_part, part * 4);
     }
     if (!ok) return fail(GLSU_ERR_ALLOC, "surrogate: device allocation failed");
@@ -197,14 +193,13 @@ int SurNet::backward(const void *d_z, const void *d_target)
     GLSU_TRY(raise_smem_limit((const void *)sur_dw_small_kernel<32, 2>, sur_dw_small_smem(64, 32, 2)));
     sur_dw_small_kernel<2, 32><<<nbs, 288, sur_dw_small_smem(dil[7], 2, 32), stream>>>(d_dh, d_act[6], B, H, W,
                                                                                        dil[7], d_part);
-    sur_reduce_kernel<<<(kSurL7Params + 31) / 32, sur_reduce_threads(nbs), 0, stream>>>(d_part, nbs, kSurL7Params,
+    sur_reduce_kernel<false><<<(kSurL7Params + 31) / 32, sur_reduce_threads(nbs), 0, stream>>>(d_part, nbs, kSurL7Params,
                                                                      d_grad + sur_layer_offset(7));
     sur_l7_bwd_kernel<<<g, 256, 0, stream>>>(d_dh, d_act[6], B, H, W, dil[7], d_w7r, d_g[0]);
     GLSU_CUDA_TRY(cudaGetLastError());
-    const size_t npx = (size_t)B * H * W;
     for (int l = 6; l >= 1; l--) {
-        uint16_t *gl = d_g[(6 - l) & 1], *gprev = d_g[(7 - l) & 1];
-        // weights on the tensor cores, bias on CUDA cores, each summed over its partials in a fixed order
+        uint16_t *gprev = d_g[(7 - l) & 1];
+        // weights and biases, summed over the CTAs' partials in a fixed order
         SurWgradArgs wa;
         wa.B = B;
         wa.H = H;
@@ -214,9 +209,8 @@ int SurNet::backward(const void *d_z, const void *d_target)
         wa.err = d_err;
         int nblk = 0;
         GLSU_TRY(launch_sur_wgrad(map_fwd[l], map_g[(6 - l) & 1], wa, stream, &nblk));
-        sur_reduce_kernel<<<9216 / 32, sur_reduce_threads(nblk), 0, stream>>>(d_part, nblk, 9216, d_grad + sur_layer_offset(l));
-        sur_db32_kernel<<<ndb, 256, 0, stream>>>(gl, npx, kSurDbPix, d_part);
-        sur_reduce_kernel<<<1, sur_reduce_threads(ndb), 0, stream>>>(d_part, ndb, 32, d_grad + sur_layer_offset(l) + 9216);
+        sur_reduce_kernel<true><<<kWgCols / 32, sur_reduce_threads(nblk), 0, stream>>>(d_part, nblk, kWgCols,
+                                                                                       d_grad + sur_layer_offset(l));
         GLSU_CUDA_TRY(cudaGetLastError());
         SurConvArgs a;
         a.B = B;
@@ -234,7 +228,7 @@ int SurNet::backward(const void *d_z, const void *d_target)
     // layer 0: weight gradient from g0 (in d_g[0] after six swaps) and the input
     sur_dw_small_kernel<32, 2><<<nbs, 288, sur_dw_small_smem(dil[0], 32, 2), stream>>>(d_g[0], z, B, H, W, dil[0],
                                                                                        d_part);
-    sur_reduce_kernel<<<(kSurL0Params + 31) / 32, sur_reduce_threads(nbs), 0, stream>>>(d_part, nbs, kSurL0Params, d_grad);
+    sur_reduce_kernel<false><<<(kSurL0Params + 31) / 32, sur_reduce_threads(nbs), 0, stream>>>(d_part, nbs, kSurL0Params, d_grad);
     GLSU_CUDA_TRY(cudaGetLastError());
     return GLSU_OK;
 }
@@ -442,12 +436,10 @@ namespace glsu {
 int sur_wgrad32_once(const void *d_g, const void *d_in, int batch, int width, int height, int dilation, float *h_dw,
                      cudaStream_t s)
 {
-    const size_t n = (size_t)batch * height * width;
-    const int ndb = (int)((n + kSurDbPix - 1) / kSurDbPix);
     float *d_part = nullptr, *d_out = nullptr;
     int *d_err = nullptr;
     int rc = GLSU_OK;
-    const size_t part = std::max<size_t>((size_t)device_sm_count() * 9216, (size_t)ndb * 32);
+    const size_t part = (size_t)device_sm_count() * kWgCols;
     if (cudaMalloc(&d_part, part * 4) != cudaSuccess || cudaMalloc(&d_out, kSurL32Params * 4) != cudaSuccess ||
         cudaMalloc(&d_err, 4) != cudaSuccess)
         rc = fail(GLSU_ERR_ALLOC, "allocation failed");
@@ -466,9 +458,7 @@ int sur_wgrad32_once(const void *d_g, const void *d_in, int batch, int width, in
         int nblk = 0;
         rc = launch_sur_wgrad(tma, tmg, wa, s, &nblk);
         if (rc == GLSU_OK) {
-            sur_reduce_kernel<<<9216 / 32, sur_reduce_threads(nblk), 0, s>>>(d_part, nblk, 9216, d_out);
-            sur_db32_kernel<<<ndb, 256, 0, s>>>((const uint16_t *)d_g, n, kSurDbPix, d_part);
-            sur_reduce_kernel<<<1, sur_reduce_threads(ndb), 0, s>>>(d_part, ndb, 32, d_out + 9216);
+            sur_reduce_kernel<true><<<kWgCols / 32, sur_reduce_threads(nblk), 0, s>>>(d_part, nblk, kWgCols, d_out);
             if (cudaGetLastError() != cudaSuccess) rc = fail(GLSU_ERR_CUDA, "weight-gradient launch failed");
         }
     }

@@ -50,6 +50,7 @@
 #include <atomic>
 #include <cmath>
 
+#include "dpra_ls_ff.cuh"
 #include "glsu_internal.cuh"
 #include "ptx_sm103.cuh"
 
@@ -88,6 +89,9 @@ __device__ __forceinline__ void sur_unit(float yr, float yi, float &orr, float &
 }
 
 __device__ __forceinline__ float bf2f(uint16_t v) { return __uint_as_float((uint32_t)v << 16); }
+
+// A float-float sum in FP32; where the sum is not finite its low part is NaN.
+__device__ __forceinline__ float ff_value(ff a) { return isfinite(a.hi) ? a.hi + a.lo : a.hi; }
 
 __device__ __forceinline__ uint32_t pack_bf2(float lo, float hi)
 {
@@ -598,10 +602,13 @@ __global__ void __launch_bounds__(256) sur_l7_bwd_kernel(const float2 *__restric
 // gradient w.r.t. the layer's output,
 //   dW[co][ci][ky][kx] = sum_{b, y', x} g[b, y' - (ky-1) d, x, co] a[b, y', x + (kx-1) d, ci]
 // (y' = y + (ky-1) d: each activation row y' meets the gradient rows y' + d,
-// y', y' - d).  A work item is one 128-pixel segment of one activation row.
-// Per 16 pixels one MMA D[M = 128][N = 96] += A[M][K = 16] B[K][N]:
-//   A: the three gradient rows, M = ky * 32 + co (a zeroed fourth block pads
-//      M to 128);
+// y', y' - d).  A work item is one 128-pixel segment of `rows` activation rows
+// d apart, taken downwards: with its rows + 2 gradient rows in consecutive
+// slots (slot j: the top activation row + d - j d) the i-th activation row
+// meets the three slots i, i + 1, i + 2.  Per 16 pixels and activation row one
+// MMA D[M = 128][N = 96] += A[M][K = 16] B[K][N]:
+//   A: those three gradient rows, M = ky * 32 + co (the slot after them pads M
+//      to 128, zeros behind the last: lanes 96-127 are not read);
 //   B: the activation row, N = kx * 32 + ci, its three kx blocks d pixels
 //      apart.
 // Both operands are the pixel-major rows that TMA writes with 64-byte
@@ -609,15 +616,52 @@ __global__ void __launch_bounds__(256) sur_l7_bwd_kernel(const float2 *__restric
 // direction), pixels 64 bytes apart and 8-pixel groups 512 bytes apart (K),
 // the 32-channel blocks LBO apart (the gradient slot stride for A, 64 d bytes
 // for B).  The accumulator stays in TMEM across all of a CTA's items; the
-// epilogue writes it once as the CTA's partial, part[blk][co][ci][ky*3+kx].
-constexpr int kWgStages = 4;
+// epilogue writes it once as the CTA's partial, part[blk][t = ky*3+kx][ci][co]
+// with co along the lanes.
+// The bias gradient, the sum of g, comes from the same shared-memory rows: the
+// four warps that wait for the epilogue add up each item's centre slots,
+// compensated from item to item, into part[blk][9216 + co].
+// What bounds it is the L2 traffic of the operands, (2 rows + 2) row segments
+// per `rows`: one row an item, as this kernel had, reads every gradient row
+// three times.  A training pass at 16 x 256 x 256: 1522 us with one row an item,
+// a bias pass over g of 21 us a layer and FP64 reductions, 1212 us as here.
+constexpr int kWgMaxRows = 4;
+constexpr int kWgMaxStages = 4;
 constexpr int kWgSlot = 128 * 64;          // one 128-pixel gradient row segment
 constexpr int kWgPad = 16 * 1024;          // slack after the stages
+constexpr int kWgTail = 1024;              // barriers and the bias sums of four warps
+constexpr int kWgSmemMax = 232448;
 constexpr uint32_t kWgTmemCols = 128;
+constexpr int kWgCols = kSurL32Params;     // columns of a partial: weights, then biases
 
 __host__ __device__ inline int sur_wgrad_act_bytes(int dil) { return ((128 + 2 * dil) * 64 + 1023) & ~1023; }
-__host__ __device__ inline int sur_wgrad_stage_bytes(int dil) { return 4 * kWgSlot + sur_wgrad_act_bytes(dil); }
-inline int sur_wgrad_smem_bytes(int dil) { return kWgStages * sur_wgrad_stage_bytes(dil) + kWgPad + 256; }
+// gradient slots, the zero slot, activation rows
+__host__ __device__ inline int sur_wgrad_stage_bytes(int dil, int rows)
+{
+    return (rows + 3) * kWgSlot + rows * sur_wgrad_act_bytes(dil);
+}
+inline int sur_wgrad_stages(int dil, int rows)
+{
+    return std::min(kWgMaxStages, (kWgSmemMax - kWgPad - kWgTail) / sur_wgrad_stage_bytes(dil, rows));
+}
+inline int sur_wgrad_smem_bytes(int dil, int rows)
+{
+    return sur_wgrad_stages(dil, rows) * sur_wgrad_stage_bytes(dil, rows) + kWgPad + kWgTail;
+}
+// First activation row of an item (0 .. rows) that is inside the image; those
+// above it in the item's order are neither loaded nor multiplied.
+__host__ __device__ inline int sur_wgrad_first(int top, int H, int dil, int rows)
+{
+    if (top < H) return 0;
+    const int j = (top - H) / dil + 1;
+    return j < rows ? j : rows;
+}
+// Items of a batch: rows of a residue class mod d, `rows` at a time, by segments.
+inline int sur_wgrad_items(int B, int H, int W, int dil, int rows)
+{
+    const int classes = std::min(dil, H), chain = (H + dil - 1) / dil;
+    return B * classes * ((chain + rows - 1) / rows) * ((W + 127) / 128);
+}
 
 // MN-major operand in the 64-byte swizzle layout: 32-element blocks `lbo`
 // bytes apart, 8-row (K) groups 512 bytes apart.
@@ -629,101 +673,180 @@ __device__ __forceinline__ uint64_t umma_desc_mn_sw64(uint32_t saddr, uint32_t l
 
 struct SurWgradArgs {
     int B = 0, H = 0, W = 0, dil = 1;
-    float *part = nullptr;  // [gridDim.x][9216]
+    float *part = nullptr;  // [gridDim.x][kWgCols]
     int *err = nullptr;
 };
 
 __global__ void __launch_bounds__(256, 1) sur_wgrad_tc_kernel(const __grid_constant__ CUtensorMap tma,
                                                               const __grid_constant__ CUtensorMap tmg,
-                                                              SurWgradArgs a, int nitems)
+                                                              SurWgradArgs a, int nitems, int rows, int stages)
 {
     extern __shared__ __align__(1024) unsigned char sm[];
-    const int stage_bytes = sur_wgrad_stage_bytes(a.dil);
-    uint64_t *full = reinterpret_cast<uint64_t *>(sm + kWgStages * stage_bytes + kWgPad);
-    uint64_t *sfree = full + kWgStages;
-    uint64_t *done = sfree + kWgStages;
+    const int stage_bytes = sur_wgrad_stage_bytes(a.dil, rows), act_bytes = sur_wgrad_act_bytes(a.dil);
+    uint64_t *full = reinterpret_cast<uint64_t *>(sm + stages * stage_bytes + kWgPad);
+    uint64_t *sfree = full + kWgMaxStages;
+    uint64_t *done = sfree + kWgMaxStages;
     uint32_t *tslot = reinterpret_cast<uint32_t *>(done + 1);
+    float *bsum = reinterpret_cast<float *>(full) + 64;  // [4 warps][32]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nsx = (a.W + 127) / 128;
     if (tid == 0) {
-        for (int s = 0; s < kWgStages; s++) {
+        for (int s = 0; s < stages; s++) {
             mbar_init(&full[s], 1);
-            mbar_init(&sfree[s], 1);
+            mbar_init(&sfree[s], 1 + 4);  // the MMAs' commit and the four bias warps
         }
         mbar_init(done, 1);
         fence_mbar_init();
     }
     if (warp == 0) tmem_alloc(tslot, kWgTmemCols);
-    // the fourth gradient block of every stage stays zero: it pads M to 128
-    for (int s = 0; s < kWgStages; s++)
+    // the slot after the gradient rows of every stage stays zero
+    for (int s = 0; s < stages; s++)
         for (int e = tid; e < kWgSlot / 16; e += 256)
-            reinterpret_cast<uint4 *>(sm + s * stage_bytes + 3 * kWgSlot)[e] = make_uint4(0, 0, 0, 0);
+            reinterpret_cast<uint4 *>(sm + s * stage_bytes + (rows + 2) * kWgSlot)[e] = make_uint4(0, 0, 0, 0);
     fence_proxy_async_smem();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tslot;
+    // every MMA accumulates
+    if (warp >= 4) {
+        const float z[32] = {};
+        for (int c = 0; c < 96; c += 32) tmem_st32(tmem + ((uint32_t)((warp - 4) * 32) << 16) + c, z);
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+
+    // the top (last) activation row of an item
+    const int classes = min(a.dil, a.H), groups = ((a.H + a.dil - 1) / a.dil + rows - 1) / rows;
+    auto top_of = [&](int item) {
+        const int i = item / nsx;
+        return i % classes + ((i / classes % groups + 1) * rows - 1) * a.dil;
+    };
 
     if (warp == 0 && elect_one()) {
-        // ---- producer: per item three gradient rows and one activation row ----
-        uint32_t g = 0;
+        // ---- producer: per item up to rows + 2 gradient rows and `rows` activation rows ----
+        uint32_t s = 0, lap = 0;
         bool ok = true;
-        for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x, g++) {
-            const int sx = item % nsx, yb = item / nsx, y = yb % a.H, b = yb / a.H;
-            const int s = g % kWgStages;
-            if (g >= (uint32_t)kWgStages && !mbar_wait_bounded(&sfree[s], ((g / kWgStages) - 1) & 1)) {
+        for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
+            const int sx = item % nsx, b = item / nsx / classes / groups, top = top_of(item);
+            const int j0 = sur_wgrad_first(top, a.H, a.dil, rows);
+            const uint32_t bytes =
+                (uint32_t)(rows + 2 - j0) * kWgSlot + (uint32_t)((rows - j0) * (128 + 2 * a.dil)) * 64;
+            if (lap > 0 && !mbar_wait_bounded(&sfree[s], (lap - 1) & 1)) {
                 ok = false;
                 break;
             }
-            unsigned char *st = sm + s * stage_bytes;
-            mbar_expect_tx(&full[s], 3u * kWgSlot + (uint32_t)(128 + 2 * a.dil) * 64);
+            unsigned char *st = sm + s * stage_bytes, *sa = st + (rows + 3) * kWgSlot;
+            mbar_expect_tx(&full[s], bytes);
             // rows outside the image arrive as zeros
-            tma_load_4d(st, &tmg, &full[s], 0, sx * 128, y + a.dil, b);
-            tma_load_4d(st + kWgSlot, &tmg, &full[s], 0, sx * 128, y, b);
-            tma_load_4d(st + 2 * kWgSlot, &tmg, &full[s], 0, sx * 128, y - a.dil, b);
-            tma_load_4d(st + 4 * kWgSlot, &tma, &full[s], 0, sx * 128 - a.dil, y, b);
+            for (int j = j0; j < rows + 2; j++)
+                tma_load_4d(st + j * kWgSlot, &tmg, &full[s], 0, sx * 128, top + (1 - j) * a.dil, b);
+            for (int j = j0; j < rows; j++)
+                tma_load_4d(sa + j * act_bytes, &tma, &full[s], 0, sx * 128 - a.dil, top - j * a.dil, b);
+            if (++s == (uint32_t)stages) {
+                s = 0;
+                lap++;
+            }
         }
         if (!ok) atomicExch(a.err, GLSU_ERR_TIMEOUT);
-        for (uint32_t j = g > (uint32_t)kWgStages ? g - kWgStages : 0; j < g; j++)
-            mbar_wait_bounded(&full[j % kWgStages], (j / kWgStages) & 1);
+        // no copy is in flight when the CTA ends: each stage's last one
+        for (uint32_t j = 0; j < (uint32_t)stages; j++) {
+            const uint32_t uses = lap + (j < s ? 1 : 0);
+            if (uses > 0) mbar_wait_bounded(&full[j], (uses - 1) & 1);
+        }
     } else if (warp == 1 && elect_one()) {
         // ---- MMA issuer ----
         const uint32_t idesc = umma_idesc_bf16(128, 96) | (1u << 15) | (1u << 16);  // A and B MN-major
-        uint32_t g = 0, acc = 0;
+        uint32_t s = 0, lap = 0;
         bool ok = true;
-        for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x, g++) {
-            const int s = g % kWgStages;
-            if (!mbar_wait_bounded(&full[s], (g / kWgStages) & 1)) {
+        for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
+            if (!mbar_wait_bounded(&full[s], lap & 1)) {
                 ok = false;
                 break;
             }
             tc_fence_after();
-            const uint32_t gb = smem_u32(sm + s * stage_bytes), ab = gb + 4 * kWgSlot;
+            const int j0 = sur_wgrad_first(top_of(item), a.H, a.dil, rows);
+            const uint32_t st = smem_u32(sm + s * stage_bytes);
+            uint32_t gb = st + j0 * kWgSlot, ab = st + (rows + 3) * kWgSlot + j0 * act_bytes;
+            for (int j = j0; j < rows; j++, gb += kWgSlot, ab += act_bytes) {
 #pragma unroll
-            for (int k = 0; k < 8; k++) {
-                umma_bf16(tmem, umma_desc_mn_sw64(gb + k * 1024, kWgSlot),
-                          umma_desc_mn_sw64(ab + k * 1024, (uint32_t)a.dil * 64), idesc, acc);
-                acc = 1;
+                for (int k = 0; k < 8; k++)
+                    umma_bf16(tmem, umma_desc_mn_sw64(gb + k * 1024, kWgSlot),
+                              umma_desc_mn_sw64(ab + k * 1024, (uint32_t)a.dil * 64), idesc, 1);
             }
             umma_commit(&sfree[s]);
+            if (++s == (uint32_t)stages) {
+                s = 0;
+                lap++;
+            }
         }
         if (!ok) atomicExch(a.err, GLSU_ERR_TIMEOUT);
         umma_commit(done);  // every MMA has completed before the epilogue reads and TMEM is released
         mbar_wait_bounded(done, 0);
-    } else if (warp >= 4 && warp < 7) {
+    } else if (warp >= 4) {
+        // ---- bias sums: thread = (8-channel group, pixel lane 0..31) of the centre rows ----
+        const int cg = tid & 3, pl = (tid - 128) >> 2;
+        ff acc[8];
+#pragma unroll
+        for (int c = 0; c < 8; c++) acc[c] = {0.f, 0.f};
+        uint32_t s = 0, lap = 0;
+        bool ok = true;
+        for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
+            if (!__all_sync(0xffffffffu, mbar_wait_bounded(&full[s], lap & 1))) {
+                ok = false;
+                break;
+            }
+            float sum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            for (int j = sur_wgrad_first(top_of(item), a.H, a.dil, rows) + 1; j <= rows; j++) {
+                const unsigned char *row = sm + s * stage_bytes + j * kWgSlot;
+                float v[4][8];
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const int px = pl + 32 * i;
+                    unpack8(*reinterpret_cast<const uint4 *>(row + px * 64 + ((cg ^ ((px >> 1) & 3)) << 4)), v[i]);
+                }
+#pragma unroll
+                for (int c = 0; c < 8; c++) sum[c] += (v[0][c] + v[1][c]) + (v[2][c] + v[3][c]);
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sfree[s]);
+#pragma unroll
+            for (int c = 0; c < 8; c++) {
+                const ff t = ff_two_sum(acc[c].hi, sum[c]);
+                acc[c] = {t.hi, acc[c].lo + t.lo};
+            }
+            if (++s == (uint32_t)stages) {
+                s = 0;
+                lap++;
+            }
+        }
+        // the 8 lanes of a channel group, then the four warps in order
+#pragma unroll
+        for (int c = 0; c < 8; c++) {
+#pragma unroll
+            for (int o = 4; o < 32; o <<= 1) {
+                const ff t = ff_two_sum(acc[c].hi, __shfl_xor_sync(0xffffffffu, acc[c].hi, o));
+                acc[c] = {t.hi, acc[c].lo + __shfl_xor_sync(0xffffffffu, acc[c].lo, o) + t.lo};
+            }
+            if (lane < 4) bsum[(warp - 4) * 32 + cg * 8 + c] = ff_value(acc[c]);
+        }
+        asm volatile("bar.sync 1, 128;" ::: "memory");
         // ---- epilogue: lanes 0-95 (ky = warp - 4, co = lane) -> the CTA's partial ----
-        const int ky = warp - 4;
-        const bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(done, 0));
+        float *pp = a.part + (size_t)blockIdx.x * kWgCols + lane;
+        if (warp == 7) pp[9216] = ((bsum[lane] + bsum[32 + lane]) + bsum[64 + lane]) + bsum[96 + lane];
+        if (!__all_sync(0xffffffffu, mbar_wait_bounded(done, 0))) ok = false;
         if (!ok && lane == 0) atomicExch(a.err, GLSU_ERR_TIMEOUT);
         tc_fence_after();
-        const bool any = blockIdx.x < nitems;
-        float *pp = a.part + (size_t)blockIdx.x * 9216 + (size_t)lane * 288;
+        if (warp < 7) {
+            const int ky = warp - 4;
 #pragma unroll
-        for (int kx = 0; kx < 3; kx++) {
-            float v[32];
-            tmem_ld32(tmem + ((uint32_t)(ky * 32) << 16) + (uint32_t)(kx * 32), v);
+            for (int kx = 0; kx < 3; kx++) {
+                float v[32];
+                tmem_ld32(tmem + ((uint32_t)(ky * 32) << 16) + (uint32_t)(kx * 32), v);
 #pragma unroll
-            for (int ci = 0; ci < 32; ci++) pp[ci * 9 + ky * 3 + kx] = (any && ok) ? v[ci] : 0.f;
+                for (int ci = 0; ci < 32; ci++) pp[((ky * 3 + kx) * 32 + ci) * 32] = ok ? v[ci] : 0.f;
+            }
         }
     }
     tc_fence_before();
@@ -732,44 +855,24 @@ __global__ void __launch_bounds__(256, 1) sur_wgrad_tc_kernel(const __grid_const
     if (warp == 0) tmem_dealloc(tmem, kWgTmemCols);
 }
 
+// Rows of an item: as many as fit two stages and still leave an item for every
+// SM (a small image is faster by a row at a time than with SMs idle).
 int launch_sur_wgrad(const CUtensorMap &tma, const CUtensorMap &tmg, const SurWgradArgs &a, cudaStream_t s,
                      int *nblocks)
 {
     if (a.dil < 1 || a.dil > 64) return fail(GLSU_ERR_INVALID, "surrogate dilation must be 1..64");
-    GLSU_TRY(raise_smem_limit((const void *)sur_wgrad_tc_kernel, sur_wgrad_smem_bytes(64),
-                              (int)cudaSharedmemCarveoutMaxShared));
-    const int items = a.B * a.H * ((a.W + 127) / 128);
-    const int grid = std::max(1, std::min(items, device_sm_count()));
-    sur_wgrad_tc_kernel<<<grid, 256, sur_wgrad_smem_bytes(a.dil), s>>>(tma, tmg, a, items);
+    GLSU_TRY(raise_smem_limit((const void *)sur_wgrad_tc_kernel, kWgSmemMax, (int)cudaSharedmemCarveoutMaxShared));
+    const int sms = device_sm_count();
+    int rows = kWgMaxRows;
+    while (rows > 1 && (sur_wgrad_stages(a.dil, rows) < 2 || sur_wgrad_items(a.B, a.H, a.W, a.dil, rows) < sms))
+        rows /= 2;
+    const int items = sur_wgrad_items(a.B, a.H, a.W, a.dil, rows);
+    const int grid = std::min(items, sms);
+    sur_wgrad_tc_kernel<<<grid, 256, sur_wgrad_smem_bytes(a.dil, rows), s>>>(tma, tmg, a, items, rows,
+                                                                             sur_wgrad_stages(a.dil, rows));
     GLSU_CUDA_TRY(cudaGetLastError());
     *nblocks = grid;
     return GLSU_OK;
-}
-
-// Bias gradient of a 32-channel layer: part[blk][c] = sum of g[p][c] over
-// the block's pixel range.  Thread = (pixel lane 0..63, 8-channel group) with
-// 16-byte loads; the 64 lanes' sums are added in lane order.
-__global__ void __launch_bounds__(256) sur_db32_kernel(const uint16_t *__restrict__ g, size_t n, int per_block,
-                                                       float *__restrict__ part)
-{
-    __shared__ float s[64][33];
-    const int cg = threadIdx.x & 3, pl = threadIdx.x >> 2;
-    const size_t p0 = (size_t)blockIdx.x * per_block;
-    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (size_t p = p0 + pl; p < p0 + per_block && p < n; p += 64) {
-        float v[8];
-        unpack8(reinterpret_cast<const uint4 *>(g + p * 32)[cg], v);
-#pragma unroll
-        for (int i = 0; i < 8; i++) acc[i] += v[i];
-    }
-#pragma unroll
-    for (int i = 0; i < 8; i++) s[pl][cg * 8 + i] = acc[i];
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        float t = s[0][threadIdx.x];
-        for (int k = 1; k < 64; k++) t += s[k][threadIdx.x];
-        part[(size_t)blockIdx.x * 32 + threadIdx.x] = t;
-    }
 }
 
 // Layer 0 (g: BF16 32 channels, input z: complex) and layer 7 (g = dh:
@@ -889,29 +992,51 @@ int sur_dw_small_blocks(int B, int H, int W)
 }
 int sur_dw_small_smem(int dil, int cout, int cin) { return (kDsSeg * cout + 3 * (kDsSeg + 2 * dil) * cin) * 4; }
 
-// Deterministic column sums of per-block partials: out[c] = sum_b part[b][c].
-// A block takes 32 columns; its warps (blockDim.x / 32 of them) sum every
-// nw-th partial in FP64, then the warps' sums are added in warp order.
+// Deterministic column sums of per-block partials: sum_b part[b][c].  A block
+// takes 32 columns; its warps (blockDim.x / 32 of them) sum every nw-th
+// partial, then warp 0 adds the warps' sums in order, all in float-float (two
+// FP64 operations an element made it FP64-bound).  WGRAD: the columns are
+// those of sur_wgrad_tc_kernel, [t][ci][co] then the biases; out has the
+// parameters' order W[co][ci][t], b[co].
+template <bool WGRAD>
 __global__ void __launch_bounds__(1024) sur_reduce_kernel(const float *__restrict__ part, int nblocks, int ncols,
                                                           float *__restrict__ out)
 {
-    __shared__ double s[32][32];
+    __shared__ float2 s[32][32];
     const int nw = blockDim.x >> 5, w = threadIdx.x >> 5, l = threadIdx.x & 31;
     const int c = blockIdx.x * 32 + l;
-    double acc = 0;
-    if (c < ncols)
-        for (int b = w; b < nblocks; b += nw) acc += part[(size_t)b * ncols + c];
-    s[w][l] = acc;
+    ff acc = {0.f, 0.f};
+    if (c < ncols) {
+        int b = w;
+        for (; b + 3 * nw < nblocks; b += 4 * nw) {
+            float v[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) v[i] = part[(size_t)(b + i * nw) * ncols + c];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const ff t = ff_two_sum(acc.hi, v[i]);
+                acc = {t.hi, acc.lo + t.lo};
+            }
+        }
+        for (; b < nblocks; b += nw) {
+            const ff t = ff_two_sum(acc.hi, part[(size_t)b * ncols + c]);
+            acc = {t.hi, acc.lo + t.lo};
+        }
+    }
+    s[w][l] = make_float2(acc.hi, acc.lo);
     __syncthreads();
     if (w == 0 && c < ncols) {
-        double t = s[0][l];
-        for (int k = 1; k < nw; k++) t += s[k][l];
-        out[c] = (float)t;
+        for (int k = 1; k < nw; k++) {
+            const ff t = ff_two_sum(acc.hi, s[k][l].x);
+            acc = {t.hi, acc.lo + s[k][l].y + t.lo};
+        }
+        const int o = !WGRAD || c >= 9216 ? c : (c & 31) * 288 + ((c >> 5) & 31) * 9 + (c >> 10);
+        out[o] = ff_value(acc);
     }
 }
 
 // Threads of a reduction: more warps when there are many partials.
-inline int sur_reduce_threads(int nblocks) { return nblocks >= 1024 ? 1024 : nblocks >= 256 ? 512 : 256; }
+inline int sur_reduce_threads(int nblocks) { return nblocks >= 1024 ? 1024 : nblocks >= 128 ? 512 : 256; }
 
 __global__ void sur_sum_kernel(const double *__restrict__ part, int n, double *__restrict__ out)
 {
