@@ -64,7 +64,7 @@ int SurNet::init(int batch, int width, int height, const int *dilations, bool tr
              A((void **)&d_v, kSurParams * 4) && A((void **)&d_lpart, (size_t)kSurPixBlocks * 8) &&
              A((void **)&d_y, n * 8) &&
              A((void **)&d_loss, 8);
-        nbs = sur_dw_small_blocks(B, H, W);
+        nbs = sur_narrow_blocks(B, H, W);
         const size_t part = std::max<size_t>((size_t)device_sm_count() * kWgCols, (size_t)nbs * kSurL0Params);
         ok = ok && A((void **)&d_part, part * 4);
     }
@@ -183,19 +183,16 @@ int SurNet::backward(const void *d_z, const void *d_target)
     if (!training) return fail(GLSU_ERR_INVALID, "surrogate handle was not created for training");
     const float2 *z = (const float2 *)d_z;
     GLSU_TRY(hidden(z));
-    const int g = rows_grid();
     GLSU_TRY(last(z, nullptr, d_y));
     sur_l7_loss_kernel<<<kSurPixBlocks, 256, 0, stream>>>(d_y, (const float2 *)d_target, (size_t)B * H * W, d_out,
                                                           d_dh, d_lpart, loss_scale);
     sur_sum_kernel<<<1, 32, 0, stream>>>(d_lpart, kSurPixBlocks, d_loss);
     // layer 7: weight gradient and dL/da6 (masked)
-    GLSU_TRY(raise_smem_limit((const void *)sur_dw_small_kernel<2, 32>, sur_dw_small_smem(64, 2, 32)));
-    GLSU_TRY(raise_smem_limit((const void *)sur_dw_small_kernel<32, 2>, sur_dw_small_smem(64, 32, 2)));
-    sur_dw_small_kernel<2, 32><<<nbs, 288, sur_dw_small_smem(dil[7], 2, 32), stream>>>(d_dh, d_act[6], B, H, W,
-                                                                                       dil[7], d_part);
-    sur_reduce_kernel<false><<<(kSurL7Params + 31) / 32, sur_reduce_threads(nbs), 0, stream>>>(d_part, nbs, kSurL7Params,
-                                                                     d_grad + sur_layer_offset(7));
-    sur_l7_bwd_kernel<<<g, 256, 0, stream>>>(d_dh, d_act[6], B, H, W, dil[7], d_w7r, d_g[0]);
+    const int nwi = sur_narrow_items(B, H, W);
+    sur_narrow_bwd_kernel<true><<<nbs, 256, sur_narrow_smem(dil[7]), stream>>>(d_act[6], d_dh, B, H, W, dil[7], nwi,
+                                                                               d_w7r, d_g[0], d_part);
+    sur_reduce_kernel<false><<<(kSurL7Params + 31) / 32, sur_reduce_threads(nbs), 0, stream>>>(
+        d_part, nbs, kSurL7Params, d_grad + sur_layer_offset(7));
     GLSU_CUDA_TRY(cudaGetLastError());
     for (int l = 6; l >= 1; l--) {
         uint16_t *gprev = d_g[(7 - l) & 1];
@@ -226,9 +223,10 @@ int SurNet::backward(const void *d_z, const void *d_target)
         GLSU_TRY(launch_sur_conv(map_bwd[l], map_bwd_out[l], a, stream));
     }
     // layer 0: weight gradient from g0 (in d_g[0] after six swaps) and the input
-    sur_dw_small_kernel<32, 2><<<nbs, 288, sur_dw_small_smem(dil[0], 32, 2), stream>>>(d_g[0], z, B, H, W, dil[0],
-                                                                                       d_part);
-    sur_reduce_kernel<false><<<(kSurL0Params + 31) / 32, sur_reduce_threads(nbs), 0, stream>>>(d_part, nbs, kSurL0Params, d_grad);
+    sur_narrow_bwd_kernel<false><<<nbs, 256, sur_narrow_smem(dil[0]), stream>>>(d_g[0], z, B, H, W, dil[0], nwi,
+                                                                                nullptr, nullptr, d_part);
+    sur_reduce_kernel<false><<<(kSurL0Params + 31) / 32, sur_reduce_threads(nbs), 0, stream>>>(d_part, nbs,
+                                                                                               kSurL0Params, d_grad);
     GLSU_CUDA_TRY(cudaGetLastError());
     return GLSU_OK;
 }

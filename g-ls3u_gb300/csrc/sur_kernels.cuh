@@ -554,47 +554,6 @@ __global__ void __launch_bounds__(256) sur_l7_loss_kernel(const float2 *__restri
     if (tid == 0) part[blockIdx.x] = red[0];
 }
 
-// dL/da6 through layer 7, masked by ReLU'(a6): g6[p][ci] = [a6 > 0] *
-// sum_t sum_co w7[co][ci][t] dh[p - off_t][co]
-__global__ void __launch_bounds__(256) sur_l7_bwd_kernel(const float2 *__restrict__ dh,
-                                                         const uint16_t *__restrict__ a6, int B, int H, int W,
-                                                         int dil, const float *__restrict__ w7,
-                                                         uint16_t *__restrict__ g6)
-{
-    __shared__ float ws[576];
-    for (int e = threadIdx.x; e < 576; e += 256) ws[e] = w7[e];
-    __syncthreads();
-    for (int row = blockIdx.x; row < B * H; row += gridDim.x)
-    for (int x = threadIdx.x; x < W; x += 256) {
-        const int y = row % H;
-        const size_t p = (size_t)row * W + x;
-        const size_t img = (size_t)(row - y) * W;
-        float acc[32];
-#pragma unroll
-        for (int c = 0; c < 32; c++) acc[c] = 0.f;
-#pragma unroll
-        for (int t = 0; t < 9; t++) {
-            const int yy = y - (t / 3 - 1) * dil, xx = x - (t % 3 - 1) * dil;
-            if (yy < 0 || yy >= H || xx < 0 || xx >= W) continue;
-            const float2 d = dh[img + (size_t)yy * W + xx];
-#pragma unroll
-            for (int c = 0; c < 32; c++) acc[c] = fmaf(ws[c * 9 + t], d.x, fmaf(ws[288 + c * 9 + t], d.y, acc[c]));
-        }
-        const uint4 *ap = reinterpret_cast<const uint4 *>(a6 + p * 32);
-        uint4 *op = reinterpret_cast<uint4 *>(g6 + p * 32);
-#pragma unroll
-        for (int g = 0; g < 4; g++) {
-            float av[8];
-            unpack8(ap[g], av);
-#pragma unroll
-            for (int i = 0; i < 8; i++)
-                if (!(av[i] > 0.f)) acc[8 * g + i] = 0.f;
-            op[g] = make_uint4(pack_bf2(acc[8 * g], acc[8 * g + 1]), pack_bf2(acc[8 * g + 2], acc[8 * g + 3]),
-                               pack_bf2(acc[8 * g + 4], acc[8 * g + 5]), pack_bf2(acc[8 * g + 6], acc[8 * g + 7]));
-        }
-    }
-}
-
 // ---------------------------------------------------------------------------
 // weight gradients
 // ---------------------------------------------------------------------------
@@ -875,122 +834,176 @@ int launch_sur_wgrad(const CUtensorMap &tma, const CUtensorMap &tmg, const SurWg
     return GLSU_OK;
 }
 
-// Layer 0 (g: BF16 32 channels, input z: complex) and layer 7 (g = dh:
-// complex, input a6: BF16 32 channels) on CUDA cores: a block takes 8 rows
-// of one 64-pixel segment, staging per row the gradient and the three input
-// rows (with the dilated halo) in shared memory as FP32 (16-byte loads of
-// 8 BF16 channels); thread c < 288 owns (tap t = c / 32, j = c % 32) and
-// accumulates the two weights that pair j with both channels of the
-// 2-channel side.  part[blk][co][ci][t] then the biases part[blk][576 + co].
-constexpr int kDsSeg = 64, kDsRows = 8;
+// Backward of the two layers between 2 and 32 channels, on CUDA cores.  With u
+// the 32-channel BF16 side and v the complex side, both sum
+//   dW[t] += u[p] v[p + s off_t],  off_t = ((ky-1) d, (kx-1) d),
+// layer 0 (LAST false) with u = g0, v = z, s = +1, layer 7 with u = a6, v = dh,
+// s = -1; layer 7 also needs, of the same values,
+//   g6[p][ci] = [a6 > 0] * sum_t sum_co w7[co][ci][t] dh[p - off_t][co].
+// A CTA takes items of kNwRows rows of a 128-pixel segment: v's rows y - d, y,
+// y + d with the dilated halo are staged in shared memory, u is read once,
+// straight from global memory, a warp's step being PX pixels with CH channels
+// a lane.  Of the nine v[] that a lane reads (one 8-byte broadcast load each,
+// for PX pixels), it makes 18 CH FMAs, 36 CH with g6: the FMA rate bounds
+// both.  A thread's FP32 chain is at most kNwItems x 32 products long.
+// part[blk][co][ci][t], then the biases part[blk][576 + co].
+// 16 x 256 x 256 (under the profiler): 116 + 111 us of layer 7 and 91 us of
+// layer 0 with weights, values and gradients all read from shared memory, 108
+// and 62 us as here.
+constexpr int kNwSeg = 128, kNwRows = 4, kNwItems = 16, kNwWarps = 8;
+constexpr int kNwCols = 576 + 32;  // columns of a partial, at most
 
-__device__ __forceinline__ void store8(float *d, const float *v)
+template <bool LAST>
+__global__ void __launch_bounds__(32 * kNwWarps, 2)
+    sur_narrow_bwd_kernel(const uint16_t *__restrict__ wide, const float2 *__restrict__ narrow, int B, int H, int W,
+                          int dil, int nitems, const float *__restrict__ w7, uint16_t *__restrict__ g6,
+                          float *__restrict__ part)
 {
-    reinterpret_cast<float4 *>(d)[0] = make_float4(v[0], v[1], v[2], v[3]);
-    reinterpret_cast<float4 *>(d)[1] = make_float4(v[4], v[5], v[6], v[7]);
-}
+    constexpr int CH = LAST ? 2 : 4, PX = CH, LP = 32 / PX;  // channels a lane, pixels a step, lanes a pixel
+    constexpr int SPR = kNwSeg / (kNwWarps * PX);            // steps a row
+    constexpr int Q = 4;                                     // steps whose u are loaded together
+    static_assert(SPR % Q == 0, "whole groups a row");
+    extern __shared__ __align__(16) float2 vs[];  // [3][kNwRows][SW]; at the end the warps' sums
+    const int SW = kNwSeg + 2 * dil;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, cl = lane % LP, hp = lane / LP;
+    const int nsx = (W + kNwSeg - 1) / kNwSeg, nby = (H + kNwRows - 1) / kNwRows;
+    float w[LAST ? 9 : 1][2][CH];
+    if (LAST) {
+#pragma unroll
+        for (int t = 0; t < 9; t++)
+#pragma unroll
+            for (int c = 0; c < CH; c++) {
+                w[t][0][c] = w7[(cl * CH + c) * 9 + t];
+                w[t][1][c] = w7[288 + (cl * CH + c) * 9 + t];
+            }
+    }
+    float acc[9][2][CH], bias[LAST ? 2 : CH];
+#pragma unroll
+    for (int t = 0; t < 9; t++)
+#pragma unroll
+        for (int c = 0; c < CH; c++) acc[t][0][c] = acc[t][1][c] = 0.f;
+#pragma unroll
+    for (int c = 0; c < (LAST ? 2 : CH); c++) bias[c] = 0.f;
 
-template <int COUT, int CIN>
-__global__ void __launch_bounds__(288) sur_dw_small_kernel(const void *__restrict__ gptr,
-                                                           const void *__restrict__ inptr, int B, int H, int W,
-                                                           int dil, float *__restrict__ part)
-{
-    static_assert((COUT == 2 && CIN == 32) || (COUT == 32 && CIN == 2), "layer 0 or layer 7");
-    extern __shared__ __align__(16) float dss[];
-    const int SW = kDsSeg + 2 * dil;
-    float *gs = dss;                      // [64][COUT]
-    float *is = gs + kDsSeg * COUT;       // [3][SW][CIN]
-    const int nsx = (W + kDsSeg - 1) / kDsSeg, nby = (H + kDsRows - 1) / kDsRows;
-    int item = blockIdx.x;
-    const int sx = item % nsx;
-    item /= nsx;
-    const int by = item % nby, b = item / nby;
-    const int x0 = sx * kDsSeg;
-    const int tid = threadIdx.x, t = tid >> 5, j = tid & 31;
-    const int ky = t / 3, kx = t % 3;
-    float acc0 = 0.f, acc1 = 0.f, bacc = 0.f;
-    const float zero8[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int yy = 0; yy < kDsRows; yy++) {
-        const int y = by * kDsRows + yy;
-        if (y >= H) break;
+    for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
+        const int sx = item % nsx, by = item / nsx % nby, b = item / nsx / nby;
+        const int x0 = sx * kNwSeg, y0 = by * kNwRows, nr = min(kNwRows, H - y0);
+        const size_t img = (size_t)b * H * W;
+        auto load = [&](int q, uint32_t(&u)[Q][CH / 2]) {  // group q of the item; zeros right of the image
+#pragma unroll
+            for (int i = 0; i < Q; i++) {
+                const int y = y0 + q / (SPR / Q), x = x0 + ((q % (SPR / Q) * Q + i) * kNwWarps + warp) * PX + hp;
+                const uint32_t *src =
+                    reinterpret_cast<const uint32_t *>(wide + (img + (size_t)y * W + x) * 32 + cl * CH);
+                if constexpr (CH == 2) {
+                    u[i][0] = x < W ? *src : 0;
+                } else {
+                    const uint2 v = x < W ? *reinterpret_cast<const uint2 *>(src) : make_uint2(0, 0);
+                    u[i][0] = v.x;
+                    u[i][1] = v.y;
+                }
+            }
+        };
+        uint32_t cur[Q][CH / 2], nxt[Q][CH / 2];
+        load(0, cur);
         __syncthreads();
-        if (COUT == 32) {  // g0: 4 x 16 bytes a pixel
-            for (int e = tid; e < kDsSeg * 4; e += 288) {
-                const int px = e >> 2, c8 = e & 3, x = x0 + px;
-                float v[8];
-                if (x < W) unpack8(reinterpret_cast<const uint4 *>(gptr)[(((size_t)b * H + y) * W + x) * 4 + c8], v);
-                store8(gs + px * 32 + c8 * 8, x < W ? v : zero8);
-            }
-        } else {  // dh: one complex a pixel
-            for (int px = tid; px < kDsSeg; px += 288) {
-                const int x = x0 + px;
-                float2 v = make_float2(0.f, 0.f);
-                if (x < W) v = reinterpret_cast<const float2 *>(gptr)[((size_t)b * H + y) * W + x];
-                gs[px * 2] = v.x;
-                gs[px * 2 + 1] = v.y;
-            }
-        }
-        if (CIN == 32) {  // a6: 4 x 16 bytes a pixel
-            for (int e = tid; e < 3 * SW * 4; e += 288) {
-                const int c8 = e & 3, rest = e >> 2, px = rest % SW, r = rest / SW;
-                const int ys = y + (r - 1) * dil, xs = x0 - dil + px;
-                const bool in = ys >= 0 && ys < H && xs >= 0 && xs < W;
-                float v[8];
-                if (in) unpack8(reinterpret_cast<const uint4 *>(inptr)[(((size_t)b * H + ys) * W + xs) * 4 + c8], v);
-                store8(is + (r * SW + px) * 32 + c8 * 8, in ? v : zero8);
-            }
-        } else {  // z: one complex a pixel
-            for (int e = tid; e < 3 * SW; e += 288) {
-                const int px = e % SW, r = e / SW;
-                const int ys = y + (r - 1) * dil, xs = x0 - dil + px;
-                float2 v = make_float2(0.f, 0.f);
-                if (ys >= 0 && ys < H && xs >= 0 && xs < W)
-                    v = reinterpret_cast<const float2 *>(inptr)[((size_t)b * H + ys) * W + xs];
-                is[(r * SW + px) * 2] = v.x;
-                is[(r * SW + px) * 2 + 1] = v.y;
-            }
+        for (int e = tid; e < 3 * kNwRows * SW; e += 32 * kNwWarps) {
+            const int r = e / SW, px = e - r * SW;
+            const int ys = y0 + r % kNwRows + (r / kNwRows - 1) * dil, xs = x0 - dil + px;
+            const bool in = ys >= 0 && ys < H && xs >= 0 && xs < W;
+            vs[e] = in ? narrow[img + (size_t)ys * W + xs] : make_float2(0.f, 0.f);
         }
         __syncthreads();
-        const float *ir = is + (size_t)(ky * SW + kx * dil) * CIN;
-        if (COUT == 2) {  // layer 7: j = ci, the two output channels
-#pragma unroll 8
-            for (int px = 0; px < kDsSeg; px++) {
-                const float iv = ir[px * CIN + j];
-                const float2 gv = reinterpret_cast<const float2 *>(gs)[px];
-                acc0 = fmaf(gv.x, iv, acc0);
-                acc1 = fmaf(gv.y, iv, acc1);
+        const int nq = nr * (SPR / Q);
+        for (int q = 0; q < nq; q++) {
+            if (q + 1 < nq) load(q + 1, nxt);
+#pragma unroll
+            for (int i = 0; i < Q; i++) {
+                const int rr = q / (SPR / Q), px = ((q % (SPR / Q) * Q + i) * kNwWarps + warp) * PX + hp;
+                const float2 *vp = vs + rr * SW + px;
+                float a[CH];
+#pragma unroll
+                for (int c = 0; c < CH; c++)
+                    a[c] = __uint_as_float(c & 1 ? cur[i][c / 2] & 0xFFFF0000u : cur[i][c / 2] << 16);
+                float g[CH];
+#pragma unroll
+                for (int c = 0; c < CH; c++) g[c] = 0.f;
+#pragma unroll
+                for (int t = 0; t < 9; t++) {
+                    const int k = LAST ? 8 - t : t;  // the staged neighbour: rows k / 3, columns k % 3
+                    const float2 v = vp[(k / 3) * kNwRows * SW + (k % 3) * dil];
+#pragma unroll
+                    for (int c = 0; c < CH; c++) {
+                        acc[t][0][c] = fmaf(v.x, a[c], acc[t][0][c]);
+                        acc[t][1][c] = fmaf(v.y, a[c], acc[t][1][c]);
+                        if (LAST) g[c] = fmaf(w[t][0][c], v.x, fmaf(w[t][1][c], v.y, g[c]));
+                    }
+                    if (LAST && t == 4) {
+                        bias[0] += v.x;
+                        bias[1] += v.y;
+                    }
+                }
+                if (!LAST) {
+#pragma unroll
+                    for (int c = 0; c < CH; c++) bias[c] += a[c];
+                }
+                if constexpr (LAST) {
+                    const int x = x0 + px;
+                    if (x < W)
+                        *reinterpret_cast<uint32_t *>(g6 + (img + (size_t)(y0 + rr) * W + x) * 32 + cl * 2) =
+                            pack_bf2(a[0] > 0.f ? g[0] : 0.f, a[1] > 0.f ? g[1] : 0.f);
+                }
             }
-            if (tid < 2)
-                for (int px = 0; px < kDsSeg; px++) bacc += gs[px * 2 + tid];
-        } else {  // layer 0: j = co, the two input channels
-#pragma unroll 8
-            for (int px = 0; px < kDsSeg; px++) {
-                const float gv = gs[px * 32 + j];
-                const float2 iv = reinterpret_cast<const float2 *>(ir)[px];
-                acc0 = fmaf(gv, iv.x, acc0);
-                acc1 = fmaf(gv, iv.y, acc1);
-            }
-            if (tid < 32)
-                for (int px = 0; px < kDsSeg; px++) bacc += gs[px * 32 + tid];
+#pragma unroll
+            for (int i = 0; i < Q; i++)
+#pragma unroll
+                for (int c = 0; c < CH / 2; c++) cur[i][c] = nxt[i][c];
         }
     }
-    float *pp = part + (size_t)blockIdx.x * (COUT * CIN * 9 + COUT);
-    if (COUT == 2) {
-        pp[(0 * 32 + j) * 9 + t] = acc0;
-        pp[(1 * 32 + j) * 9 + t] = acc1;
-        if (tid < 2) pp[576 + tid] = bacc;
-    } else {
-        pp[(j * 2 + 0) * 9 + t] = acc0;
-        pp[(j * 2 + 1) * 9 + t] = acc1;
-        if (tid < 32) pp[576 + tid] = bacc;
+    // the lanes of a channel, then the warps in order
+    __syncthreads();
+    float *red = reinterpret_cast<float *>(vs) + warp * kNwCols;
+    auto lanes = [&](float x) {
+#pragma unroll
+        for (int o = LP; o < 32; o <<= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        return x;
+    };
+#pragma unroll
+    for (int t = 0; t < 9; t++)
+#pragma unroll
+        for (int k = 0; k < 2; k++)
+#pragma unroll
+            for (int c = 0; c < CH; c++) {
+                const float x = lanes(acc[t][k][c]);
+                const int ch = cl * CH + c;
+                if (hp == 0) red[(LAST ? k * 32 + ch : ch * 2 + k) * 9 + t] = x;
+            }
+#pragma unroll
+    for (int c = 0; c < (LAST ? 2 : CH); c++) {
+        const float x = lanes(bias[c]);
+        if (hp == 0 && (!LAST || cl == 0)) red[576 + (LAST ? c : cl * CH + c)] = x;
+    }
+    __syncthreads();
+    constexpr int cols = LAST ? kSurL7Params : kSurL0Params;
+    const float *rp = reinterpret_cast<const float *>(vs);
+    for (int c = tid; c < cols; c += 32 * kNwWarps) {
+        float x = rp[c];
+        for (int k = 1; k < kNwWarps; k++) x += rp[k * kNwCols + c];
+        part[(size_t)blockIdx.x * cols + c] = x;
     }
 }
 
-int sur_dw_small_blocks(int B, int H, int W)
+int sur_narrow_items(int B, int H, int W) { return B * ((H + kNwRows - 1) / kNwRows) * ((W + kNwSeg - 1) / kNwSeg); }
+// One wave of CTAs, more where a thread's chain would pass kNwItems items.
+int sur_narrow_blocks(int B, int H, int W)
 {
-    return B * ((H + kDsRows - 1) / kDsRows) * ((W + kDsSeg - 1) / kDsSeg);
+    const int items = sur_narrow_items(B, H, W);
+    return std::min(items, std::max(2 * device_sm_count(), (items + kNwItems - 1) / kNwItems));
 }
-int sur_dw_small_smem(int dil, int cout, int cin) { return (kDsSeg * cout + 3 * (kDsSeg + 2 * dil) * cin) * 4; }
+int sur_narrow_smem(int dil)
+{
+    return std::max(3 * kNwRows * (kNwSeg + 2 * dil) * 8, kNwWarps * kNwCols * 4);
+}
 
 // Deterministic column sums of per-block partials: sum_b part[b][c].  A block
 // takes 32 columns; its warps (blockDim.x / 32 of them) sum every nw-th

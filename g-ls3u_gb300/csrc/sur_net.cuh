@@ -25,7 +25,7 @@ struct SurNet {
     float2 *d_dh = nullptr, *d_out = nullptr, *d_y = nullptr;  // y = z + h7 before the renormalisation
     float *d_grad = nullptr, *d_m = nullptr, *d_v = nullptr, *d_part = nullptr;
     double *d_lpart = nullptr, *d_loss = nullptr;
-    int nbs = 0, adam_t = 0;  // blocks of the small weight-gradient kernels
+    int nbs = 0, adam_t = 0;  // blocks of the backward kernels of layers 0 and 7
     int conv_ctas_per_sm = 0;  // cap of the tensor-core layers' CTAs per SM (0: none)
     float loss_scale = 1.f;    // training loss weight min(loss_scale |target|, 1)
     int *d_err = nullptr;

@@ -69,6 +69,8 @@ def _shift(x, dy, dx):
     """x [B,H,W,C] -> x[:, y+dy, x+dx] with zeros outside."""
     B, H, W, C = x.shape
     out = np.zeros_like(x)
+    if abs(dy) >= H or abs(dx) >= W:
+        return out
     ys, yd = max(0, dy), max(0, -dy)
     xs, xd = max(0, dx), max(0, -dx)
     out[:, yd:H - ys, xd:W - xs] = x[:, ys:H - yd, xs:W - xd]

@@ -1,9 +1,11 @@
 """Kernels of the training pass at their edges: items of four, two and one rows
-of the tensor-core weight gradient, with rows outside the image."""
+of the tensor-core weight gradient, with rows outside the image, and the
+backward kernels of the two layers between 2 and 32 channels."""
 import numpy as np
 import pytest
 
-from test_surrogate import _bf16_bits, _from_bits, _torch
+from oracle import surrogate as S
+from test_surrogate import _bf16_bits, _from_bits, _net_case, _torch
 
 pytestmark = pytest.mark.gpu
 
@@ -37,3 +39,27 @@ def test_weight_gradient_rows_per_item(glsu, shape, dil):
     rdb = g.sum((0, 1, 2))
     assert np.abs(dw - ref).max() <= 1e-5 * np.abs(ref).max()
     assert np.abs(db - rdb).max() <= 1e-6 * np.abs(rdb).max()
+
+
+# heights and widths around the 4-row, 128-pixel items of the first and last
+# layer's backward kernels, and dilations that leave whole taps outside
+@pytest.mark.parametrize("shape,first,last", [((1, 1, 1), 1, 1), ((1, 5, 3), 2, 64), ((2, 4, 128), 64, 1),
+                                              ((2, 9, 129), 1, 3), ((1, 7, 260), 33, 1)])
+def test_narrow_layer_gradients(glsu, shape, first, last):
+    """Against the oracle with the same BF16 rounding points; what differs is
+    FP32 against FP64 sums, and through them a rare BF16 step of one value, as
+    in the test of the whole network: 2e-2 of a layer's gradient."""
+    dil = [first, 2, 4, 8, 4, 2, 1, last]
+    torch, p, z, t = _net_case(glsu, *shape, 11)
+    net = glsu.Surrogate(shape[0], shape[2], shape[1], dil, training=True)
+    net.params = p
+    dz, dt = torch.from_numpy(z).cuda(), torch.from_numpy(t).cuda()
+    _, g = net.backward(dz.data_ptr(), dt.data_ptr(), want_grad=True)
+    _, again = net.backward(dz.data_ptr(), dt.data_ptr(), want_grad=True)
+    net.close()
+    assert np.array_equal(g, again)
+    _, rg = S.loss_and_grad(p, z.astype(np.complex128), t.astype(np.complex128), dil)
+    offs = np.cumsum([0] + [co * ci * 9 + co for co, ci in S.SIZES])
+    for k in (0, 6, 7):
+        a, b = g[offs[k]:offs[k + 1]].astype(np.float64), rg[offs[k]:offs[k + 1]]
+        assert np.linalg.norm(a - b) <= 2e-2 * np.linalg.norm(b)
