@@ -189,7 +189,7 @@ int SurNet::backward(const void *d_z, const void *d_target)
     sur_sum_kernel<<<1, 32, 0, stream>>>(d_lpart, kSurPixBlocks, d_loss);
     // layer 7: weight gradient and dL/da6 (masked)
     const int nwi = sur_narrow_items(B, H, W);
-    sur_narrow_bwd_kernel<true><<<nbs, 256, sur_narrow_smem(dil[7]), stream>>>(d_act[6], d_dh, B, H, W, dil[7], nwi,
+    sur_narrow_bwd_kernel<true><<<nbs, kNwThreads, sur_narrow_smem(dil[7]), stream>>>(d_act[6], d_dh, B, H, W, dil[7], nwi,
                                                                                d_w7r, d_g[0], d_part);
     sur_reduce_kernel<false><<<(kSurL7Params + 31) / 32, sur_reduce_threads(nbs), 0, stream>>>(
         d_part, nbs, kSurL7Params, d_grad + sur_layer_offset(7));
@@ -223,7 +223,7 @@ int SurNet::backward(const void *d_z, const void *d_target)
         GLSU_TRY(launch_sur_conv(map_bwd[l], map_bwd_out[l], a, stream));
     }
     // layer 0: weight gradient from g0 (in d_g[0] after six swaps) and the input
-    sur_narrow_bwd_kernel<false><<<nbs, 256, sur_narrow_smem(dil[0]), stream>>>(d_g[0], z, B, H, W, dil[0], nwi,
+    sur_narrow_bwd_kernel<false><<<nbs, kNwThreads, sur_narrow_smem(dil[0]), stream>>>(d_g[0], z, B, H, W, dil[0], nwi,
                                                                                 nullptr, nullptr, d_part);
     sur_reduce_kernel<false><<<(kSurL0Params + 31) / 32, sur_reduce_threads(nbs), 0, stream>>>(d_part, nbs,
                                                                                                kSurL0Params, d_grad);

@@ -841,123 +841,147 @@ int launch_sur_wgrad(const CUtensorMap &tma, const CUtensorMap &tmg, const SurWg
 // s = -1; layer 7 also needs, of the same values,
 //   g6[p][ci] = [a6 > 0] * sum_t sum_co w7[co][ci][t] dh[p - off_t][co].
 // A CTA takes items of kNwRows rows of a 128-pixel segment: v's rows y - d, y,
-// y + d with the dilated halo are staged in shared memory, u is read once,
-// straight from global memory, a warp's step being PX pixels with CH channels
-// a lane.  Of the nine v[] that a lane reads (one 8-byte broadcast load each,
-// for PX pixels), it makes 18 CH FMAs, 36 CH with g6: the FMA rate bounds
-// both.  A thread's FP32 chain is at most kNwItems x 32 products long.
+// y + d with the dilated halo are staged in shared memory as (x, x, y, y), u
+// is read once, straight from global memory (the next item's asked into L2
+// meanwhile), a warp's step being PX pixels with CH channels a lane.  The nine
+// v that a lane reads (one 16-byte broadcast load each, for PX pixels) meet
+// its channel pairs in 9 CH packed FMAs, 18 CH with g6.  What bounds it is
+// latency: accumulators and weights take 72 registers, so three CTAs of four
+// warps with 168 registers a thread fit, and the FMA pipe is busy 40 % of the
+// time.  A thread's FP32 chain is at most 512 products long.
 // part[blk][co][ci][t], then the biases part[blk][576 + co].
 // 16 x 256 x 256 (under the profiler): 116 + 111 us of layer 7 and 91 us of
-// layer 0 with weights, values and gradients all read from shared memory, 108
-// and 62 us as here.
-constexpr int kNwSeg = 128, kNwRows = 4, kNwItems = 16, kNwWarps = 8;
+// layer 0 with weights, values and gradients all read from shared memory; 108
+// and 62 us with scalar FMAs and two CTAs of eight warps at 128 registers; the
+// training pass 1060 us with those, 1036 us as here (1061 with packed FMAs
+// alone, 1048 with four rows an item).
+constexpr int kNwSeg = 128, kNwRows = 2, kNwWarps = 4, kNwThreads = 32 * kNwWarps;
+constexpr int kNwCtas = 3;                            // per SM
+constexpr int kNwItems = 8 * kNwWarps / kNwRows;      // of a CTA, at most: chains of 512 products
 constexpr int kNwCols = 576 + 32;  // columns of a partial, at most
 
+__device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 template <bool LAST>
-__global__ void __launch_bounds__(32 * kNwWarps, 2)
+__global__ void __launch_bounds__(kNwThreads, kNwCtas)
     sur_narrow_bwd_kernel(const uint16_t *__restrict__ wide, const float2 *__restrict__ narrow, int B, int H, int W,
                           int dil, int nitems, const float *__restrict__ w7, uint16_t *__restrict__ g6,
                           float *__restrict__ part)
 {
     constexpr int CH = LAST ? 2 : 4, PX = CH, LP = 32 / PX;  // channels a lane, pixels a step, lanes a pixel
-    constexpr int SPR = kNwSeg / (kNwWarps * PX);            // steps a row
+    constexpr int C2 = CH / 2, ST = kNwWarps * PX;           // channel pairs; pixels between a warp's steps
     constexpr int Q = 4;                                     // steps whose u are loaded together
-    static_assert(SPR % Q == 0, "whole groups a row");
-    extern __shared__ __align__(16) float2 vs[];  // [3][kNwRows][SW]; at the end the warps' sums
+    constexpr int GR = kNwSeg / (ST * Q);                    // such groups a row
+    extern __shared__ __align__(16) float4 vs[];  // (x, x, y, y) [3][kNwRows][SW]; at the end the warps' sums
     const int SW = kNwSeg + 2 * dil;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, cl = lane % LP, hp = lane / LP;
     const int nsx = (W + kNwSeg - 1) / kNwSeg, nby = (H + kNwRows - 1) / kNwRows;
-    float w[LAST ? 9 : 1][2][CH];
+    float2 w[LAST ? 9 : 1][2];
     if (LAST) {
 #pragma unroll
         for (int t = 0; t < 9; t++)
 #pragma unroll
-            for (int c = 0; c < CH; c++) {
-                w[t][0][c] = w7[(cl * CH + c) * 9 + t];
-                w[t][1][c] = w7[288 + (cl * CH + c) * 9 + t];
-            }
+            for (int k = 0; k < 2; k++)
+                w[t][k] = make_float2(w7[k * 288 + cl * 18 + t], w7[k * 288 + cl * 18 + 9 + t]);
     }
-    float acc[9][2][CH], bias[LAST ? 2 : CH];
+    float2 acc[9][2][C2], bias[C2];
 #pragma unroll
-    for (int t = 0; t < 9; t++)
+    for (int c = 0; c < C2; c++) {
+        bias[c] = make_float2(0.f, 0.f);
 #pragma unroll
-        for (int c = 0; c < CH; c++) acc[t][0][c] = acc[t][1][c] = 0.f;
-#pragma unroll
-    for (int c = 0; c < (LAST ? 2 : CH); c++) bias[c] = 0.f;
+        for (int t = 0; t < 9; t++) acc[t][0][c] = acc[t][1][c] = make_float2(0.f, 0.f);
+    }
+    const int off = warp * PX + hp;  // the lane's pixel in a step
 
     for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
         const int sx = item % nsx, by = item / nsx % nby, b = item / nsx / nby;
         const int x0 = sx * kNwSeg, y0 = by * kNwRows, nr = min(kNwRows, H - y0);
-        const size_t img = (size_t)b * H * W;
-        auto load = [&](int q, uint32_t(&u)[Q][CH / 2]) {  // group q of the item; zeros right of the image
+        const size_t img = (size_t)b * H * W, first = (img + (size_t)y0 * W + x0 + off) * 32 + cl * CH;
+        const int left = W - x0 - off;  // the lane's steps at or beyond it lie right of the image
+        auto load = [&](int q, uint32_t(&u)[Q][C2]) {
+            const uint16_t *src = wide + first + ((size_t)(q / GR) * W + q % GR * (Q * ST)) * 32;
 #pragma unroll
             for (int i = 0; i < Q; i++) {
-                const int y = y0 + q / (SPR / Q), x = x0 + ((q % (SPR / Q) * Q + i) * kNwWarps + warp) * PX + hp;
-                const uint32_t *src =
-                    reinterpret_cast<const uint32_t *>(wide + (img + (size_t)y * W + x) * 32 + cl * CH);
-                if constexpr (CH == 2) {
-                    u[i][0] = x < W ? *src : 0;
+                const bool in = (q % GR * Q + i) * ST < left;
+                if constexpr (C2 == 1) {
+                    u[i][0] = in ? *reinterpret_cast<const uint32_t *>(src + i * ST * 32) : 0;
                 } else {
-                    const uint2 v = x < W ? *reinterpret_cast<const uint2 *>(src) : make_uint2(0, 0);
+                    const uint2 v = in ? *reinterpret_cast<const uint2 *>(src + i * ST * 32) : make_uint2(0, 0);
                     u[i][0] = v.x;
-                    u[i][1] = v.y;
+                    u[i][C2 - 1] = v.y;
                 }
             }
         };
-        uint32_t cur[Q][CH / 2], nxt[Q][CH / 2];
+        uint32_t cur[Q][C2], nxt[Q][C2];
         load(0, cur);
         __syncthreads();
-        for (int e = tid; e < 3 * kNwRows * SW; e += 32 * kNwWarps) {
-            const int r = e / SW, px = e - r * SW;
-            const int ys = y0 + r % kNwRows + (r / kNwRows - 1) * dil, xs = x0 - dil + px;
-            const bool in = ys >= 0 && ys < H && xs >= 0 && xs < W;
-            vs[e] = in ? narrow[img + (size_t)ys * W + xs] : make_float2(0.f, 0.f);
+        constexpr int V = 6;  // of v a thread loads together
+        for (int e0 = tid; e0 < 3 * kNwRows * SW; e0 += V * kNwThreads) {
+            float2 v[V];
+#pragma unroll
+            for (int i = 0; i < V; i++) {
+                const int e = e0 + i * kNwThreads, r = e / SW;
+                const int ys = y0 + r % kNwRows + (r / kNwRows - 1) * dil, xs = x0 - dil + e - r * SW;
+                const bool in = r < 3 * kNwRows && ys >= 0 && ys < H && xs >= 0 && xs < W;
+                v[i] = in ? narrow[img + (size_t)ys * W + xs] : make_float2(0.f, 0.f);
+            }
+#pragma unroll
+            for (int i = 0; i < V; i++)
+                if (e0 + i * kNwThreads < 3 * kNwRows * SW)
+                    vs[e0 + i * kNwThreads] = make_float4(v[i].x, v[i].x, v[i].y, v[i].y);
+        }
+        // the next item's u on its way into L2, lines of two pixels
+        if (item + gridDim.x < nitems) {
+            const int ni = item + gridDim.x, nx = ni % nsx * kNwSeg, ny = ni / nsx % nby * kNwRows;
+            const uint16_t *src = wide + (size_t)(ni / nsx / nby) * H * W * 32;
+#pragma unroll
+            for (int e = tid; e < kNwRows * kNwSeg / 2; e += kNwThreads) {
+                const int y = ny + e / (kNwSeg / 2), x = nx + e % (kNwSeg / 2) * 2;
+                if (y < H && x < W) prefetch_l2(src + ((size_t)y * W + x) * 32);
+            }
         }
         __syncthreads();
-        const int nq = nr * (SPR / Q);
+        const int nq = nr * GR;
+#pragma unroll 1
         for (int q = 0; q < nq; q++) {
             if (q + 1 < nq) load(q + 1, nxt);
+            const float4 *vr = vs + q / GR * SW + q % GR * (Q * ST) + off;
 #pragma unroll
             for (int i = 0; i < Q; i++) {
-                const int rr = q / (SPR / Q), px = ((q % (SPR / Q) * Q + i) * kNwWarps + warp) * PX + hp;
-                const float2 *vp = vs + rr * SW + px;
-                float a[CH];
+                float2 a[C2], g = make_float2(0.f, 0.f);
 #pragma unroll
-                for (int c = 0; c < CH; c++)
-                    a[c] = __uint_as_float(c & 1 ? cur[i][c / 2] & 0xFFFF0000u : cur[i][c / 2] << 16);
-                float g[CH];
-#pragma unroll
-                for (int c = 0; c < CH; c++) g[c] = 0.f;
+                for (int c = 0; c < C2; c++)
+                    a[c] = make_float2(__uint_as_float(cur[i][c] << 16),
+                                       __uint_as_float(cur[i][c] & 0xFFFF0000u));
 #pragma unroll
                 for (int t = 0; t < 9; t++) {
                     const int k = LAST ? 8 - t : t;  // the staged neighbour: rows k / 3, columns k % 3
-                    const float2 v = vp[(k / 3) * kNwRows * SW + (k % 3) * dil];
+                    const float4 v = (vr + (k / 3) * kNwRows * SW + (k % 3) * dil)[i * ST];
+                    const float2 vx = make_float2(v.x, v.y), vy = make_float2(v.z, v.w);
 #pragma unroll
-                    for (int c = 0; c < CH; c++) {
-                        acc[t][0][c] = fmaf(v.x, a[c], acc[t][0][c]);
-                        acc[t][1][c] = fmaf(v.y, a[c], acc[t][1][c]);
-                        if (LAST) g[c] = fmaf(w[t][0][c], v.x, fmaf(w[t][1][c], v.y, g[c]));
+                    for (int c = 0; c < C2; c++) {
+                        acc[t][0][c] = __ffma2_rn(vx, a[c], acc[t][0][c]);
+                        acc[t][1][c] = __ffma2_rn(vy, a[c], acc[t][1][c]);
                     }
-                    if (LAST && t == 4) {
-                        bias[0] += v.x;
-                        bias[1] += v.y;
+                    if (LAST) {
+                        g = __ffma2_rn(w[t][0], vx, __ffma2_rn(w[t][1], vy, g));
+                        if (t == 4) bias[0] = make_float2(bias[0].x + v.x, bias[0].y + v.z);
                     }
-                }
-                if (!LAST) {
-#pragma unroll
-                    for (int c = 0; c < CH; c++) bias[c] += a[c];
                 }
                 if constexpr (LAST) {
-                    const int x = x0 + px;
-                    if (x < W)
-                        *reinterpret_cast<uint32_t *>(g6 + (img + (size_t)(y0 + rr) * W + x) * 32 + cl * 2) =
-                            pack_bf2(a[0] > 0.f ? g[0] : 0.f, a[1] > 0.f ? g[1] : 0.f);
+                    if ((q % GR * Q + i) * ST < left)
+                        *reinterpret_cast<uint32_t *>(g6 + first + ((size_t)(q / GR) * W + q % GR * (Q * ST)) * 32 +
+                                                      i * ST * 32) =
+                            pack_bf2(a[0].x > 0.f ? g.x : 0.f, a[0].y > 0.f ? g.y : 0.f);
+                } else {
+#pragma unroll
+                    for (int c = 0; c < C2; c++) bias[c] = __fadd2_rn(bias[c], a[c]);
                 }
             }
 #pragma unroll
             for (int i = 0; i < Q; i++)
 #pragma unroll
-                for (int c = 0; c < CH / 2; c++) cur[i][c] = nxt[i][c];
+                for (int c = 0; c < C2; c++) cur[i][c] = nxt[i][c];
         }
     }
     // the lanes of a channel, then the warps in order
@@ -974,19 +998,19 @@ __global__ void __launch_bounds__(32 * kNwWarps, 2)
         for (int k = 0; k < 2; k++)
 #pragma unroll
             for (int c = 0; c < CH; c++) {
-                const float x = lanes(acc[t][k][c]);
+                const float x = lanes(c & 1 ? acc[t][k][c / 2].y : acc[t][k][c / 2].x);
                 const int ch = cl * CH + c;
                 if (hp == 0) red[(LAST ? k * 32 + ch : ch * 2 + k) * 9 + t] = x;
             }
 #pragma unroll
-    for (int c = 0; c < (LAST ? 2 : CH); c++) {
-        const float x = lanes(bias[c]);
+    for (int c = 0; c < CH; c++) {
+        const float x = lanes(c & 1 ? bias[c / 2].y : bias[c / 2].x);
         if (hp == 0 && (!LAST || cl == 0)) red[576 + (LAST ? c : cl * CH + c)] = x;
     }
     __syncthreads();
     constexpr int cols = LAST ? kSurL7Params : kSurL0Params;
     const float *rp = reinterpret_cast<const float *>(vs);
-    for (int c = tid; c < cols; c += 32 * kNwWarps) {
+    for (int c = tid; c < cols; c += kNwThreads) {
         float x = rp[c];
         for (int k = 1; k < kNwWarps; k++) x += rp[k * kNwCols + c];
         part[(size_t)blockIdx.x * cols + c] = x;
@@ -998,11 +1022,11 @@ int sur_narrow_items(int B, int H, int W) { return B * ((H + kNwRows - 1) / kNwR
 int sur_narrow_blocks(int B, int H, int W)
 {
     const int items = sur_narrow_items(B, H, W);
-    return std::min(items, std::max(2 * device_sm_count(), (items + kNwItems - 1) / kNwItems));
+    return std::min(items, std::max(kNwCtas * device_sm_count(), (items + kNwItems - 1) / kNwItems));
 }
 int sur_narrow_smem(int dil)
 {
-    return std::max(3 * kNwRows * (kNwSeg + 2 * dil) * 8, kNwWarps * kNwCols * 4);
+    return std::max(3 * kNwRows * (kNwSeg + 2 * dil) * 16, kNwWarps * kNwCols * 4);  // at most 48 KB
 }
 
 // Deterministic column sums of per-block partials: sum_b part[b][c].  A block
