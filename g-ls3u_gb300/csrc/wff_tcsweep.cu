@@ -23,7 +23,8 @@
 // wy.  Per 32 rows (two K steps):
 //   A  (2 x 4 warps)  R . e^{-j wy y}, split, tcgen05.st into an A1 slot
 //   M  (2 warps)      pass 1: A1 x B into U; pass 2: A2 x B into C
-//   B  (2 x 4 warps)  U from TMEM, threshold, split, into an A2 slot
+//   B  (2 x 4 warps)  U from TMEM, threshold (in FP64 where it is close), split,
+//                     into an A2 slot
 //   C  (2 x 4 warps)  finished rows from TMEM, times e^{+j wy y}, into registers
 // The operands never pass through shared memory: tcgen05.ld .16x256b and
 // tcgen05.st .16x128b give a thread the same image column and the same rows
@@ -35,11 +36,15 @@
 // each accumulator sees the same K steps in the same order whatever the tile:
 // a row's bits do not depend on the tile height, the batch or a tile mask.
 //
-// Bound: instruction issue.  At 1024^2, sigma 10, 21 x 21 frequencies the sweep
-// takes 1.33 ms (the FFT sweep 3.18): 2.8 instructions a clock per SM, about
-// 170 per 16 x 64 block, wy and pass for the splitting and thresholding, a
-// quarter of them waiting.  Its MMAs alone would take 0.5 ms (N/2 cycles each at
-// M = 128, K = 16, A in TMEM); the DRAM is at 3%.
+// Bound: the waits between the stages, and instruction issue.  At 1024^2, sigma
+// 10, 21 x 21 frequencies the sweep takes 1.40 ms (the FFT sweep 3.18): 2.8
+// instructions a clock per SM, about 170 per 16 x 64 block, wy and pass for the
+// splitting and thresholding, a quarter of them waiting.  With nearly all of A's,
+// B's and C's arithmetic taken out 1.0 of 1.39 ms is left: the chain slot, MMAs,
+// commit, next slot.  A third A warpgroup, up to four A1 slots, filling a slot in
+// halves, skipping empty blocks and sleeping waits each left the time as it was
+// or made it longer.  The MMAs alone would take 0.5 ms (N/2 cycles each at M =
+// 128, K = 16, A in TMEM); the DRAM is at 3%.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -85,6 +90,8 @@ struct TcSeq {
     float2 *C;
     const float *thr;
     const float *kr;     // scale that R carries
+    const float *R;      // the planes that tm maps, [plane][row pair][pitch](re, re', im, im')
+    double thr_exact;    // thr_mul without what the accumulation's truncation takes
     int H, W, pitch, nfy, eys2, ncg, nty, item0;
     float thr_mul, out_mul;
 };
@@ -182,7 +189,10 @@ __device__ __forceinline__ void tie8(float *r)
 }
 
 template <int N> __device__ __forceinline__ void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
-template <int N> __device__ __forceinline__ void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void reg_dec()  // from 72
+{
+    if constexpr (N < 72) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
+}
 
 // v = (v.x, v.y) as FP16 pairs hi and lo (v.x in the lower half)
 __device__ __forceinline__ void split2(float2 v, uint32_t &hi, uint32_t &lo)
@@ -203,6 +213,43 @@ struct TcBars {
     uint32_t tmem;
 };
 static_assert(sizeof(TcBars) <= 768, "barriers");
+
+// Whether U at image row y, column x, frequency k reaches the threshold, from R
+// itself in FP64, for the values that lie within kThrBand of it, where the
+// rounding of the split products would decide.  450 random fields against 64 bits,
+// counted where one decision on the other side showed (error over 1e-6 and over
+// 1.5 times the other sweep's): the FFT sweep 4, this one 2, those shared with the
+// direct kernel; without the FP64 decisions 3 in 150.  They cost 4% of a frame
+// (1024^2: 1662 -> 1734 us).  A whole warp works on one value, its taps over the
+// lanes: one thread's loop over them made the sweep there 1.3 ms longer.  N, tb:
+// the B operand's height and its place in shared memory (its first column is the
+// taps).
+constexpr float kThrBand = 1e-5f;  // of |U|^2
+__device__ __forceinline__ bool tc_reaches(const TcSeq &q, const unsigned char *tb, int N, int s, int plane, int y,
+                                           int x, int k, float kr)
+{
+    const float *R = q.R + ((size_t)plane * ((q.H + 1) >> 1) * q.pitch + x) * 4;
+    const float *P = reinterpret_cast<const float *>(q.ey2 + (size_t)k * q.eys2 + kTcPad);
+    const int r1 = min(q.H - 1, y + s);
+    double sr = 0, si = 0;
+#pragma unroll 1
+    for (int r = max(0, y - s) + (threadIdx.x & 31); r <= r1; r += 32) {
+        const float *e = R + (size_t)(r >> 1) * q.pitch * 4 + (r & 1), *c = P + (r >> 1) * 4 + (r & 1);
+        const int n = y + s - r;
+        const __half *g = reinterpret_cast<const __half *>(tb) + (n >> 3) * 128 + (n & 7) * 8;
+        const double w = (double)(__half2float(g[0]) + __half2float(g[N * 16]));  // exact: the parts of a float
+        const double re = e[0], im = e[2], pr = c[0], pi = c[2];
+        sr += w * (re * pr - im * pi);
+        si += w * (re * pi + im * pr);
+    }
+#pragma unroll 1
+    for (int o = 16; o > 0; o >>= 1) {
+        sr += __shfl_xor_sync(0xffffffffu, sr, o);
+        si += __shfl_xor_sync(0xffffffffu, si, o);
+    }
+    const double thr = (double)*q.thr * q.thr_exact * (double)kr;
+    return sr * sr + si * si >= thr * thr;
+}
 
 // The value of lane 0, which the compiler then knows to be the warp's.
 __device__ __forceinline__ int uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
@@ -230,6 +277,7 @@ __device__ __forceinline__ void warp_wait(uint64_t *bar, uint32_t parity, bool &
 template <int RB_, int RM_, int RA_, int RT_, int RC_> struct TcCfg {
     static constexpr int RB = RB_, RM = RM_, RA = RA_, RT = RT_, RC = RC_;
     static_assert(RM + 2 * (RA + RT + RC) <= 7 * 72, "register shares");
+    static_assert(RM <= 72 && RA <= 72 && RT <= 72 && RC >= 72, "a share is given up or taken, not both");
 };
 constexpr int kThreads = 7 * 128;
 
@@ -486,7 +534,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             TcTile t;
             const TcSeq &q = tab.seq[tc_item<NS>(tab, nseq, item, list, listn, s, m, RW, t)];
             const int nfy = q.nfy, H = q.H, urow = t.ra - s + 2 * frow, nb = t.p1 - t.p0;
-            const float thr = *q.thr * q.thr_mul * *q.kr, thr2 = thr * thr;
+            const float kr = *q.kr, thr = *q.thr * q.thr_mul * kr, thr2 = thr * thr, band = kThrBand * thr2;
             for (int k = 0; k < nfy; k++) {
                 for (int i = 0; 2 * i < nb; i++, n++) {
                     if ((n & 1) != slot) {
@@ -508,6 +556,44 @@ __global__ void __launch_bounds__(kThreads, 1)
                         tie8(r[1]);
                         tmem_zero16(u);
                         const int row = urow + 16 * (t.p0 + blk);
+                        float2 a[2][2];
+                        float near = 3.402823466e38f;
+#pragma unroll
+                        for (int j = 0; j < 2; j++)
+#pragma unroll
+                            for (int h = 0; h < 2; h++) {
+                                const float2 re = make_float2(r[h][4 * j], r[h][4 * j + 1]);
+                                const float2 im = make_float2(r[h][4 * j + 2], r[h][4 * j + 3]);
+                                a[j][h] = __ffma2_rn(im, im, __fmul2_rn(re, re));
+                                const float2 d = __fadd2_rn(a[j][h], make_float2(-thr2, -thr2));
+                                near = fminf(near, fminf(fabsf(d.x), fabsf(d.y)));
+                            }
+                        if (__any_sync(0xffffffffu, near < band)) {
+                            // what lies too near is decided in FP64, value by value
+#pragma unroll 1
+                            for (int e = 0; e < 8; e++) {
+                                const int j = e >> 2, h = (e >> 1) & 1;
+                                const float2 v = j ? (h ? a[1][1] : a[1][0]) : (h ? a[0][1] : a[0][0]);
+                                const int y = row + 8 * j + (e & 1), x = t.x0 + 16 * w4 + 8 * h + fcol;
+                                const bool mine_ = fabsf((e & 1 ? v.y : v.x) - thr2) < band &&
+                                                   (unsigned)y < (unsigned)H && x < q.W;
+                                uint32_t todo = __ballot_sync(0xffffffffu, mine_);
+                                bool over = false;
+                                while (todo) {
+                                    const int src = __ffs(todo) - 1;
+                                    todo &= todo - 1;
+                                    const bool o1 = tc_reaches(q, tb, N, s, t.plane, __shfl_sync(0xffffffffu, y, src),
+                                                               __shfl_sync(0xffffffffu, x, src), k, kr);
+                                    if (lane == src) over = o1;
+                                }
+                                const float f = over ? 3.402823466e38f : -1.f;
+#pragma unroll
+                                for (int c = 0; c < 4; c++) {
+                                    if (mine_ && e == 2 * c) a[c >> 1][c & 1].x = f;
+                                    if (mine_ && e == 2 * c + 1) a[c >> 1][c & 1].y = f;
+                                }
+                            }
+                        }
 #pragma unroll
                         for (int j = 0; j < 2; j++) {
                             const int y = row + 8 * j;  // rows outside the image carry no T
@@ -516,14 +602,14 @@ __global__ void __launch_bounds__(kThreads, 1)
                             for (int h = 0; h < 2; h++) {
                                 float2 re = make_float2(r[h][4 * j], r[h][4 * j + 1]);
                                 float2 im = make_float2(r[h][4 * j + 2], r[h][4 * j + 3]);
-                                const float2 a = __ffma2_rn(im, im, __fmul2_rn(re, re));
-                                const bool k0 = in0 && a.x >= thr2, k1 = in1 && a.y >= thr2;
+                                const bool k0 = in0 && a[j][h].x >= thr2, k1 = in1 && a[j][h].y >= thr2;
                                 re = make_float2(k0 ? re.x : 0.f, k1 ? re.y : 0.f);
                                 im = make_float2(k0 ? im.x : 0.f, k1 ? im.y : 0.f);
                                 split2(__fmul2_rn(re, ts), o[h][2 * j], o[h][4 + 2 * j]);
                                 split2(__fmul2_rn(im, ts), o[h][2 * j + 1], o[h][5 + 2 * j]);
                             }
                         }
+                        __syncwarp();
                     };
                     half(2 * i);
                     if (mine > 0) wait_ok(&bar.a2free[slot], (mine - 1) & 1, ok);
@@ -688,9 +774,9 @@ double tc_cost(const WffPlan *const *plans, int n, int rb, int sms)
     return std::ceil(items / sms) * (total / items) * 0.5 + std::max(total / sms, mx) * 0.5;
 }
 
-using Tc5 = TcCfg<5, 40, 48, 56, 128>;
-using Tc4 = TcCfg<4, 40, 56, 64, 112>;
-using Tc2 = TcCfg<2, 40, 64, 64, 88>;
+using Tc5 = TcCfg<5, 40, 48, 72, 112>;
+using Tc4 = TcCfg<4, 40, 56, 72, 104>;
+using Tc2 = TcCfg<2, 40, 64, 72, 88>;
 
 template <class Cfg, int NS>
 int tc_launch(const TcTable<NS> &tab, int nseq, int nitems, int grid, const WffPlan &P, const int2 *list,
@@ -722,6 +808,7 @@ void tc_seq(TcSeq &q, const WffPlan &P, int rw, int item0)
     q.C = (float2 *)P.d_C;
     q.thr = (const float *)P.d_thr;
     q.kr = (const float *)P.d_kr;
+    q.R = (const float *)P.d_R;
     q.H = P.H;
     q.W = P.W;
     q.pitch = P.pitch;
@@ -733,7 +820,8 @@ void tc_seq(TcSeq &q, const WffPlan &P, int rw, int item0)
     // U = 2^kTapShift kr N u; T = tscale U; C = 2^kTapShift sum T
     const double taps = std::ldexp(1.0, kTapShift);
     const double shrink = kShrink * P.sy;
-    q.thr_mul = (float)(taps / P.inv_norm * (1.0 - shrink));
+    q.thr_exact = taps / P.inv_norm;
+    q.thr_mul = (float)(q.thr_exact * (1.0 - shrink));
     q.out_mul = (float)(P.inv_norm / (taps * taps * (double)P.tc_tscale) * (1.0 + 2.0 * shrink));
 }
 

@@ -96,3 +96,31 @@ def test_fft_length_by_hand_runs_the_fft_sweep(glsu):
     b, _ = _run(glsu, f, 10.0, n=5, length=True)
     assert not np.array_equal(a, b)
     assert np.abs(a - b).max() <= TOL * np.abs(b).max()
+
+
+@pytest.mark.parametrize("shape,sigma", [((41, 37), 2.0), ((150, 133), 10.0), ((163, 171), 16.0)])
+@pytest.mark.parametrize("side", [-1, 1])
+def test_threshold_close_to_every_value(glsu, oracle, shape, sigma, side):
+    """A plane wave on the grid has |U| = sum(w) for the whole window inside the
+    image, and the threshold lies 2e-6 beside it: within the band that is decided in
+    FP64, and 10 times what R's and the phasors' FP32 rounding can move |U| by
+    (about 2^-24 each, averaged over the window).  All such values pass, or none;
+    bar of the FP32 form, 1e-5 of the field."""
+    import torch
+    h, w = shape
+    y, x = np.mgrid[0:h, 0:w].astype(np.float64)
+    f = np.exp(1j * (0.25 * x - 0.5 * y)).astype(np.complex64)
+    s = int(np.floor(3 * sigma + 0.5))
+    n = np.arange(-s, s + 1)
+    g = np.exp(-n ** 2 / (2 * sigma ** 2))
+    top = g.sum() ** 2 / (g ** 2).sum()
+    p = glsu.WffParams(sigma, 0.25, 0.25, 1.0, sigma, -0.5, -0.5, 1.0, top * (1 + side * 2e-6))
+    t = torch.from_numpy(f).cuda()
+    out = torch.empty_like(t)
+    filt = glsu.WFF2(w, h, "f32", p)
+    filt.set_method(glsu.METHOD_FFT)
+    filt.run(t.data_ptr(), out.data_ptr())
+    filt.close()
+    ref, _ = oracle.wff2(f.astype(np.complex128), *p.tuple())
+    assert (np.abs(ref).max() > 0) == (side < 0)
+    assert np.abs(out.cpu().numpy() - ref).max() <= 1e-5 * max(np.abs(ref).max(), 1e-3)
