@@ -43,7 +43,6 @@ template <typename T, int S> struct WfrGeom {
     static constexpr int BOX = (sizeof(T) == 4) ? 64 : 16;   // rows per TMA box (the plan's map)
     static constexpr int NBOX = (ROWS_R + BOX - 1) / BOX;
     static constexpr int RT = NBOX * BOX;
-    static constexpr int CTAS = sizeof(T) == 4 ? 2 : 1;  // resident per SM
     static constexpr int FPC = (int)(sizeof(C2<T>) / 4);
     static constexpr uint32_t TX_BYTES = (uint32_t)(NBOX * BOX * 32 * sizeof(C2<T>));
     static constexpr size_t SMEM = sizeof(C2<T>) * (size_t)RT * 32 + 16;
@@ -58,13 +57,13 @@ __device__ __forceinline__ double mag_of_key(double k) { return k; }
 __device__ __forceinline__ float atan2_t(float y, float x) { return atan2f(y, x); }
 __device__ __forceinline__ double atan2_t(double y, double x) { return atan2(y, x); }
 
-// Bound by the FMA rate and by latency: the compiler took 243 registers when
-// let, which left one CTA of 8 warps on an SM; at 128 two fit without spills.
-// 256 x 320, sigma 10, 41 x 41 frequencies (whole WFR2): 1169 us with one CTA
-// an SM and tiles over the row pitch (384 columns), 983 us as here, tiles over
-// the width.
+// Bound by the FMA rate and by latency at 8 warps an SM (243 registers at
+// half-size 30).  Capped at 128 registers two CTAs fit, which gains nothing at
+// 256 x 320 and costs 4% at 1024^2 (159 -> 166 ms with 161 x 161 frequencies).
+// Tiles cover the width, not the row pitch: 256 x 320, sigma 10, 41 x 41
+// frequencies (whole WFR2), 1169 us with the pitch's 384 columns, 1016 us as here.
 template <typename T, int S>
-__global__ void __launch_bounds__(WfrGeom<T, S>::THREADS, WfrGeom<T, S>::CTAS)
+__global__ void __launch_bounds__(WfrGeom<T, S>::THREADS, 1)
     wfr_cols_kernel(const __grid_constant__ CUtensorMap tmR, const C2<T> *__restrict__ ex,
                     const C2<T> *__restrict__ ey, int nfy, int W, int H, int pitch, Taps<T, S> gA,
                     T *__restrict__ pabs, int *__restrict__ pk, T *__restrict__ pph, int *__restrict__ err)
