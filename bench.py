@@ -728,8 +728,8 @@ def batched_mix(glsu, torch, seed, per_size=16, fmin=10, fmax=100):
     DPRA windows 5, 7 or 9, WFF2 with 21 x 21 frequencies, FP32, frames of
     each sequence's own seeded generator (made on the GPU before each step,
     outside the timing).  The staged batch (glsu_dpra_batch_*, graph mode:
-    the FFT column sweeps of all sequences of a transform length in one
-    persistent launch) against the same sequences run one after another
+    the column sweeps of all sequences of one y-filter, or of one transform
+    length, in one persistent launch) against the same sequences run one after another
     (graph-mode handles, one frame at a time); device time per step bracketed
     by synchronisation, summed over the steps.  The two runs' final phases
     are compared bit for bit."""
@@ -1071,20 +1071,27 @@ def run_ours(args, rank, world, local):
     col_bytes = 2 * NFX * size * pitch * 8  # read R_i planes + write C_i planes (complex64)
     sm_mhz = p_clk.get("sm_mhz") or 1900.0
     fp32_peak_tflops = 152 * 128 * 2 * sm_mhz * 1e6 / 1e12
-    if p_tuning["method"] == glsu.METHOD_FFT:
+    half = int(np.floor(3 * WFF[0] + 0.5))
+    col_bound, col_peak = "fp32", fp32_peak_tflops
+    col_peak_source = "152 SMs x 128 FP32 lanes x 2 x sampled SM clock (%.0f MHz)" % sm_mhz
+    if p_tuning["method"] == glsu.METHOD_FFT and half <= 48:  # in the place of the FFT sweep
+        col_flops = float(NFX * NFY * N * 2 * (2 * half + 1) * 4)
+        col_kernel, flop_rule = "wff_tc_kernel (WFF2 column sweep on the tensor cores)", \
+            "2 column filters x (2s+1) real taps x complex; the kernel's split FP16 products are 3 times that"
+        col_bound, col_peak, col_peak_source = "tensor", bf16_peak, peak_kind
+    elif p_tuning["method"] == glsu.METHOD_FFT:
         col_flops = fft_sweep_flops(size, NFX, NFY, p_tuning["fft_length"], pitch)
         col_kernel, flop_rule = "wff_colfft_kernel (WFF2 FFT column sweep, L = %d)" % p_tuning["fft_length"], \
             "5 L log2 L per transform, 2 nfy + 2 transforms per column and wx, + 16 L per wy"
     else:
-        sx = int(np.floor(3 * WFF[0] + 0.5))
-        col_flops = float(NFX * NFY * N * 2 * (2 * sx + 1) * 2)
+        col_flops = float(NFX * NFY * N * 2 * (2 * half + 1) * 2)
         col_kernel, flop_rule = "wff_cols_kernel (WFF2 direct column sweep)", "2 column filters x (2s+1) taps x 2"
     col_s = p_st[2] * 1e-3
     fb, P = fft_model_bytes(size)
-    plain_roof = {"kernel": col_kernel, "bound": "fp32",
-                  "achieved": col_flops / col_s / 1e12, "peak": fp32_peak_tflops, "unit": "TFLOP/s",
-                  "frac": col_flops / col_s / 1e12 / fp32_peak_tflops,
-                  "peak_source": "152 SMs x 128 FP32 lanes x 2 x sampled SM clock (%.0f MHz)" % sm_mhz,
+    plain_roof = {"kernel": col_kernel, "bound": col_bound,
+                  "achieved": col_flops / col_s / 1e12, "peak": col_peak, "unit": "TFLOP/s",
+                  "frac": col_flops / col_s / 1e12 / col_peak,
+                  "peak_source": col_peak_source,
                   "algorithmic_flops_per_launch": col_flops, "flop_rule": flop_rule, "launch_ms": p_st[2],
                   "hbm_compulsory": {"bytes_per_launch": col_bytes, "achieved": col_bytes / col_s / 1e9,
                                      "peak": hbm_peak, "unit": "GB/s", "frac": col_bytes / col_s / 1e9 / hbm_peak},

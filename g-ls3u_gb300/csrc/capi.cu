@@ -1217,17 +1217,17 @@ extern "C" int glsu_dpra_batch_step(glsu_dpra *const *handles, int n, const void
 // ---------------------------------------------------------------------------
 // Staged batch (glsu_dpra_batch_*): one frame of every active sequence per
 // step, stage by stage.  Per sequence, on its own stream: the least squares
-// and the WFF2 row pass.  Then the FFT column sweeps of all sequences that
-// share a transform length as one persistent launch over their work list
-// (one launch per length, the lengths on parallel streams); sequences on the
-// direct sweep run it on their own stream.  Then per sequence the final row
+// and the WFF2 row pass.  Then the column sweeps of all sequences that share
+// a y-filter (tensor-core sweep) or a transform length (FFT sweep) as one
+// persistent launch over their work list (the classes on parallel streams);
+// sequences on the direct sweep run it on their own stream.  Then per sequence the final row
 // pass with the phase update.  The step is captured as one CUDA graph when
 // graph mode is on.
 // ---------------------------------------------------------------------------
 struct glsu_dpra_batch {
     std::vector<glsu_dpra *> h;
     cudaStream_t stream = nullptr;
-    std::vector<cudaStream_t> cls_stream;  // one per transform-length class
+    std::vector<cudaStream_t> cls_stream;  // one per class
     std::vector<cudaEvent_t> ev;           // fork/join events
     bool use_graph = false;
     bool warm = false;

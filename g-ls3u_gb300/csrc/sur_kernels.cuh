@@ -6,7 +6,7 @@
 //     x   = (Re z, Im z)                 z = exp(j dphi) of the DPRA LS stage
 //     a0  = relu(conv0(x))               2 -> 32   CUDA cores, FP32 math
 //     a_l = relu(conv_l(a_{l-1}))        32 -> 32  tcgen05, l = 1..6
-//     y   = x + conv7(a6)                32 -> 2   CUDA cores
+//     y   = x + conv7(a6)                32 -> 2   tcgen05, N padded to 16
 //     out = y / |y|                      the stand-in for WFF2(z) / |WFF2(z)|
 // Weights and activations are BF16, accumulation FP32 (TMEM for the
 // tensor-core layers).  Activations are NHWC [B][H][W][32] BF16, 64 bytes a
@@ -491,7 +491,7 @@ int launch_sur_last(const CUtensorMap &tm, const SurConvArgs &a, cudaStream_t s)
 }
 
 // ---------------------------------------------------------------------------
-// layer 0 (2 -> 32) and layer 7 (32 -> 2) on CUDA cores
+// layer 0 (2 -> 32) on CUDA cores, the training loss
 // ---------------------------------------------------------------------------
 // Layer 0 (2 -> 32, ReLU); z: complex [B][H][W].  The weights are kernel
 // parameters, so every FMA takes its weight from the parameter bank.

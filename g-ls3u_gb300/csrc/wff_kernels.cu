@@ -24,7 +24,10 @@
 //                       threshold, c = t (*)_y gy, C_i += e^{j wy_k y} c
 //   C  wff_rows_final   out = sum_i e^{j wx_i x} (C_i (*)_x gx) * scale/N
 // Kernel B holds the column tile of R_i in shared memory (loaded by TMA,
-// zero-filled outside the image) for all nfy frequencies.
+// zero-filled outside the image) for all nfy frequencies.  Other forms of B,
+// which the cost model takes where they are faster: wff_tcsweep.cu (FP32, the
+// same filters on the tensor cores), wff_colfft.cu (FP32, FFTs per column) and
+// wff_colfft64.cu (FP64, FFTs per column).
 #include <cudaTypedefs.h>
 
 #include <algorithm>

@@ -559,8 +559,8 @@ def dpra_batch_step(handles, d_frames, img_type: int):
 
 class DpraBatch:
     """Staged batch of FP32 plain-form DPRA handles (glsu_dpra_batch_*): one
-    frame of each active sequence per step, the FFT column sweeps of all
-    sequences of a transform length in one persistent launch."""
+    frame of each active sequence per step, the column sweeps of all
+    sequences of a y-filter or transform length in one persistent launch."""
 
     def __init__(self, handles, graph: bool = False):
         self._handles = list(handles)

@@ -198,7 +198,7 @@ int glsu_wff_padded_size(const glsu_wff *h, int *padded_width, int *padded_heigh
  *
  * The column sweep is always the direct kernel (GLSU_METHOD_DIRECT): its
  * output equals glsu_wff_run's bit for bit when that handle also runs the
- * direct kernel, and agrees with the FFT column sweep to FP32 rounding. */
+ * direct kernel, and agrees with the other column sweeps to FP32 rounding. */
 int glsu_wff_run_noalloc(int width, int height, const glsu_wff_params *p, const void *d_f, void *d_filtered,
                          void *cuda_stream);
 
@@ -264,12 +264,12 @@ int glsu_dpra_update_ref_phi(glsu_dpra *h);
 int glsu_dpra_batch_step(glsu_dpra *const *handles, int n, const void *const *d_frames, int img_type);
 int glsu_dpra_batch_wait(glsu_dpra *const *handles, int n);
 /* Staged batch (no counterpart in the reference): many FP32 plain-form DPRA
- * handles (any sizes, windows and WFF parameters; at most 128 per transform
- * length and launch, more are split) run one frame each per step, stage by
- * stage: per sequence on its own stream the least squares and the WFF2 row
- * pass; then the FFT column sweeps of all sequences that share a transform
- * length as one persistent launch over their (sequence, plane, column group)
- * work list, one launch per length, the lengths on parallel streams
+ * handles (any sizes, windows and WFF parameters; at most 128 per class and
+ * launch, more are split) run one frame each per step, stage by stage: per
+ * sequence on its own stream the least squares and the WFF2 row pass; then
+ * the column sweeps class by class, a class being the sequences that share a
+ * y-filter (tensor-core sweep) or a transform length (FFT sweep), each as one
+ * persistent launch over their work list, the classes on parallel streams
  * (sequences on the direct sweep run it on their own stream); then per
  * sequence the final row pass and the phase update.  Outputs equal each
  * handle's own frames bit for bit.  Each handle follows the sequence rule
