@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         for (int i = 0; i < kPairs; i++) {
             mbar_init(&bar.ufull[i], 1);
-            mbar_init(&bar.ufree[i], 4);
+            mbar_init(&bar.ufree[i], i == 0 ? 8 : 4);  // pair 0: both B warpgroups
             mbar_init(&bar.cfull[i], 1);
             mbar_init(&bar.cfree[i], 8);
         }
@@ -538,8 +538,13 @@ __global__ void __launch_bounds__(kThreads, 1)
             for (int k = 0; k < nfy; k++) {
                 for (int i = 0; 2 * i < nb; i++, n++) {
                     if ((n & 1) != slot) {
-                        // not a whole phase of a barrier behind, where a wy has one pair only
-                        if (i == 0) wait_ok(&bar.ufull[0], parity & 1, ok);
+                        // Where a wy has one pair only, this warpgroup waits for nothing of it: it
+                        // follows the pair by its phase, which it holds until it has seen it.
+                        if (i == 0) {
+                            wait_ok(&bar.ufull[0], parity & 1, ok);
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(&bar.ufree[0]);
+                        }
                         continue;
                     }
                     wait_ok(&bar.ufull[i], (parity >> i) & 1, ok);

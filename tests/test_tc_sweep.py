@@ -124,3 +124,25 @@ def test_threshold_close_to_every_value(glsu, oracle, shape, sigma, side):
     ref, _ = oracle.wff2(f.astype(np.complex128), *p.tuple())
     assert (np.abs(ref).max() > 0) == (side < 0)
     assert np.abs(out.cpu().numpy() - ref).max() <= 1e-5 * max(np.abs(ref).max(), 1e-3)
+
+
+@pytest.mark.parametrize("shape,sigma", [((5, 70), 0.4), ((16, 64), 2.0), ((31, 130), 4.0), ((163, 64), 0.5),
+                                         ((161, 200), 1.0)])
+def test_one_pair_of_blocks_a_wy(glsu, oracle, shape, sigma):
+    """Where a wy has one pair of 16-row blocks (short images, a short last
+    tile), the two thresholding warpgroups take it in turns over many wy."""
+    f = _field(shape, 7)
+    p = glsu.WffParams(2.0, -0.2, 0.2, 0.3, sigma, -1.0, 1.0, 0.01, 0.0)
+    import torch
+    t = torch.from_numpy(f).cuda()
+    w = glsu.WFF2(shape[1], shape[0], "f32", p)
+    w.set_method(glsu.METHOD_FFT)
+    outs = []
+    for _ in range(3):
+        out = torch.full_like(t, float("nan"))
+        w.run(t.data_ptr(), out.data_ptr())
+        outs.append(out.cpu().numpy())
+    w.close()
+    ref, _ = oracle.wff2(f.astype(np.complex128), *p.tuple())
+    assert np.array_equal(outs[0], outs[1]) and np.array_equal(outs[0], outs[2])
+    assert np.abs(outs[0] - ref).max() <= TOL * np.abs(ref).max()
