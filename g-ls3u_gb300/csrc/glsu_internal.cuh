@@ -223,15 +223,14 @@ struct WffPlan {
     bool unit_input = false;   // |f| <= 1 at every pixel (DPRA): the scale of R is a constant
     void *d_tctaps = nullptr;  // B operand of the banded products, hi and lo FP16 parts
     void *d_ey2 = nullptr;     // wy phasors of row pairs
-    float *d_kr = nullptr;     // [0] the power of two that R carries, [1] scratch
+    float *d_kr = nullptr;     // the power of two that R carries
     CUtensorMap tmT;           // d_R in row pairs: {4 pitch floats, (H + 1) / 2, nfx}
-    float tc_tscale = 1, tc_sum_gx = 1;
+    float tc_tscale = 1;
     bool tc_supported() const;
     int init_tc();
     void release_tc();
     bool use_tc() const { return use_colfft() && d_tctaps != nullptr && !fft_explicit; }
 };
-int launch_tc_scale(const WffPlan &P, const void *d_f, cudaStream_t s);
 int launch_tc_sweep(const WffPlan *const *plans, int n, cudaStream_t s);
 double tc_model_ms(const WffPlan &P);
 

@@ -794,10 +794,7 @@ template <typename T, int S>
 static int launch_rows_demod(const WffPlan &P, const void *d_f, cudaStream_t s)
 {
     if constexpr (sizeof(T) == 4) {
-        if (P.use_tc()) {
-            if (!P.unit_input) GLSU_TRY(launch_tc_scale(P, d_f, s));
-            return launch_rows_demod_t<T, S, true>(P, d_f, s);
-        }
+        if (P.use_tc()) return launch_rows_demod_t<T, S, true>(P, d_f, s);
     }
     return launch_rows_demod_t<T, S, false>(P, d_f, s);
 }

@@ -15,8 +15,11 @@
 // parts, x = hi + lo with |x - hi - lo| <= 2^-24 |x|, and a K step is three
 // MMAs, lo.hi + hi.lo + hi.hi, accumulated in FP32 (the dropped lo.lo is
 // 2^-24 of the product).  Powers of two keep both parts in FP16's normal
-// range: R is written by the row pass scaled to at most 2^15 (d_kr), the
-// taps by 2^6, T by tscale to at most 2^15.
+// range: R is scaled to at most 2^15, the taps by 2^6, T by tscale to at most
+// 2^15.  An input of unit modulus (DPRA) has one scale, which the row pass
+// applies (d_kr); for any other the B warps scale each column of a tile by its
+// own largest finite value, so that a large value leaves its mark, 2^-40 of
+// itself, on its own columns and tiles only.
 //
 // One CTA of seven warpgroups per SM walks a list of (plane, 64 columns, Rw
 // rows) tiles; the tile of R (Rw + 4s rows) stays in shared memory for all
@@ -80,7 +83,8 @@ constexpr int kTapShift = 6;                // taps scaled by 2^6
 // the error against 64 bits at sigma 10 goes from 5.9e-7 to 1.4e-7 of the
 // output's norm, that of the FFT sweep.
 constexpr double kShrink = 0.82e-8;
-constexpr int kSmem = kMaxChunks * kChunkBytes + kPhRing * kPhBytes + kMaxTapBytes + 768 + 1024;
+constexpr int kScaleBytes = 4 * kCols * 4;  // column scales of two tiles, column maxima by two warpgroups
+constexpr int kSmem = kMaxChunks * kChunkBytes + kPhRing * kPhBytes + kMaxTapBytes + 768 + kScaleBytes + 1024;
 static_assert(kSmem <= 227 * 1024, "column tile exceeds shared memory");
 
 // One sequence of the sweep.
@@ -205,10 +209,28 @@ __device__ __forceinline__ void split2(float2 v, uint32_t &hi, uint32_t &lo)
     lo = *reinterpret_cast<const uint32_t *>(&l);
 }
 
+__device__ __forceinline__ float finite_abs(float v)
+{
+    const float a = fabsf(v);
+    return a <= 3.402823466e38f ? a : 0.f;
+}
+// The power of two by which a column of R whose parts' largest magnitude is mx is multiplied: its
+// values times a phasor then stay below 2^15.
+__device__ __forceinline__ float column_scale(float mx)
+{
+    const int e = (int)(__float_as_uint(mx * 1.4143f) >> 23) - 126;  // below 2^e
+    return mx > 0.f ? __uint_as_float((uint32_t)(127 + min(100, 15 - e)) << 23) : 1.f;
+}
+__device__ __forceinline__ float reciprocal_pow2(float k)
+{
+    return __uint_as_float((254u << 23) - __float_as_uint(k));
+}
+
 struct TcBars {
     uint64_t rfull[kMaxChunks], rfree[kMaxChunks], phfull[kPhRing], phfree[kPhRing];
     uint64_t a1full[2], a1free[2], a2full[2], a2free[2];
     uint64_t ufull[kPairs], ufree[kPairs], cfull[kPairs], cfree[kPairs];  // per pair of blocks
+    uint64_t kfull[2], kfree[2], rscaled;  // column scales, R scaled by them
     uint64_t drain;
     uint32_t tmem;
 };
@@ -254,20 +276,28 @@ __device__ __forceinline__ bool tc_reaches(const TcSeq &q, const unsigned char *
 // The value of lane 0, which the compiler then knows to be the warp's.
 __device__ __forceinline__ int uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
 
-// Wait, once the phase is not there yet with the bounded wait.  After a
+constexpr uint32_t kTcWaitCycles = 1u << 31;
+// Bounded wait, the clock in 32 bits: short, as its copies in every role share the
+// instruction cache with the roles' loops.  After a
 // timeout (ok false) waits return at once: the roles then run to their ends,
 // within their buffers, and the results are not used.
 __device__ __forceinline__ void wait_ok(uint64_t *bar, uint32_t parity, bool &ok)
 {
-    if (ok && !mbar_try_wait(bar, parity)) ok = mbar_wait_bounded(bar, parity);
+    if (!ok) return;
+    const uint32_t t0 = (uint32_t)clock();
+    while (!mbar_try_wait(bar, parity))
+        if ((uint32_t)clock() - t0 > kTcWaitCycles) {
+            ok = false;
+            break;
+        }
 }
 
 // The same with a warp-uniform verdict.
 __device__ __forceinline__ void warp_wait(uint64_t *bar, uint32_t parity, bool &ok)
 {
     if (!ok) return;
-    bool w = mbar_try_wait(bar, parity);
-    if (!w) w = mbar_wait_bounded(bar, parity);
+    bool w = true;
+    wait_ok(bar, parity, w);
     ok = __all_sync(0xffffffffu, w);
 }
 
@@ -308,7 +338,8 @@ __device__ __forceinline__ int tc_item(const TcTable<NS> &tab, int nseq, int ite
     return k;
 }
 
-template <class Cfg, int NS>
+// UNIT: the row pass has scaled R (an input of unit modulus).
+template <class Cfg, int NS, bool UNIT>
 __global__ void __launch_bounds__(kThreads, 1)
     wff_tc_kernel(const __grid_constant__ TcTable<NS> tab, int nseq, int nitems_full, int s, int m, int N, float tscale,
                   const uint4 *__restrict__ taps, int *__restrict__ err, const int2 *__restrict__ list,
@@ -321,6 +352,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     float4 *ph = reinterpret_cast<float4 *>(Rs + kMaxChunks * kChunkBytes);
     unsigned char *tb = reinterpret_cast<unsigned char *>(ph + kPhRing * kPhPairs);
     TcBars &bar = *reinterpret_cast<TcBars *>(tb + kMaxTapBytes);
+    float(*kcol)[kCols] = reinterpret_cast<float(*)[kCols]>(tb + kMaxTapBytes + 768);  // of two tiles, in turns
+    float(*kmax)[kCols] = kcol + 2;
 
     // warp-uniform to the compiler too: the operands of the tcgen05 instructions derive from it
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31, wg = warp >> 2, w4 = warp & 3;
@@ -353,6 +386,11 @@ __global__ void __launch_bounds__(kThreads, 1)
             mbar_init(&bar.cfull[i], 1);
             mbar_init(&bar.cfree[i], 8);
         }
+        for (int i = 0; i < 2; i++) {
+            mbar_init(&bar.kfull[i], 4);
+            mbar_init(&bar.kfree[i], 8);
+        }
+        mbar_init(&bar.rscaled, 8);
         mbar_init(&bar.drain, 2);
         fence_mbar_init();
     }
@@ -418,9 +456,8 @@ __global__ void __launch_bounds__(kThreads, 1)
             const int W = N >> 4;                           // blocks of a window
             const uint32_t idesc = (1u << 4) | (8u << 24);  // FP16 x FP16 -> FP32, M = 128; N / 8 goes to bit 17
             const uint64_t bhi = umma_desc(smem_u32(tb), 128, 256), blo = umma_desc(smem_u32(tb) + N * 32, 128, 256);
-            auto issue = [&](auto pass2, uint32_t tD, uint32_t tA, uint64_t *full, uint64_t *fre, uint64_t *afull,
+            auto issue = [&](const bool second, uint32_t tD, uint32_t tA, uint64_t *full, uint64_t *fre, uint64_t *afull,
                              uint64_t *afree) {
-                constexpr bool second = decltype(pass2)::value;
                 uint32_t n = 0;                 // operand slots used
                 uint32_t parity = 0, used = 0;  // per pair of blocks: parity of its next use, used before
                 for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
@@ -457,8 +494,9 @@ __global__ void __launch_bounds__(kThreads, 1)
                     }
                 }
             };
-            if (warp == 0) issue(std::false_type{}, tU, tA1, bar.ufull, bar.ufree, bar.a1full, bar.a1free);
-            else issue(std::true_type{}, tC, tA2, bar.cfull, bar.cfree, bar.a2full, bar.a2free);
+            const bool p2 = warp == 2;
+            issue(p2, p2 ? tC : tU, p2 ? tA2 : tA1, p2 ? bar.cfull : bar.ufull, p2 ? bar.cfree : bar.ufree,
+                  p2 ? bar.a2full : bar.a1full, p2 ? bar.a2free : bar.a1free);
             if (!ok) atomicExch(err, GLSU_ERR_TIMEOUT);
             umma_commit_warp(&bar.drain);  // every MMA has completed before TMEM is released
             mbar_wait_bounded(&bar.drain, 0);
@@ -473,7 +511,11 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int item = blockIdx.x; item < nitems; item += gridDim.x, nit++) {
             TcTile t;
             const int nfy = tab.seq[tc_item<NS>(tab, nseq, item, list, listn, s, m, RW, t)].nfy;
-            for (int ch = t.q0 >> 2; ch <= (t.q1 - 1) >> 2; ch++) wait_ok(&bar.rfull[ch], nit & 1, ok);
+            if constexpr (UNIT) {
+                for (int ch = t.q0 >> 2; ch <= (t.q1 - 1) >> 2; ch++) wait_ok(&bar.rfull[ch], nit & 1, ok);
+            } else {
+                wait_ok(&bar.rscaled, nit & 1, ok);
+            }
             for (int k = 0; k < nfy; k++, nk++) {
                 wait_ok(&bar.phfull[nk % kPhRing], (nk / kPhRing) & 1, ok);
                 const float4 *P = ph + (nk % kPhRing) * kPhPairs + frow;
@@ -529,12 +571,74 @@ __global__ void __launch_bounds__(kThreads, 1)
         const uint32_t slot = wg - 3;
         const uint32_t a0 = tA2 + 32 * slot + lanes;
         const float2 ts = make_float2(tscale, tscale);
-        uint32_t n = 0, mine = 0, parity = 0;
-        for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
+        uint32_t n = 0, mine = 0, parity = 0, nit = 0;
+        for (int item = blockIdx.x; item < nitems; item += gridDim.x, nit++) {
             TcTile t;
             const TcSeq &q = tab.seq[tc_item<NS>(tab, nseq, item, list, listn, s, m, RW, t)];
             const int nfy = q.nfy, H = q.H, urow = t.ra - s + 2 * frow, nb = t.p1 - t.p0;
-            const float kr = *q.kr, thr = *q.thr * q.thr_mul * kr, thr2 = thr * thr, band = kThrBand * thr2;
+            const float kr = *q.kr, thr = *q.thr * q.thr_mul * kr;
+            float thr2[2] = {thr, thr};  // of the thread's two columns
+            if constexpr (!UNIT) {
+                // scale the tile's columns in place, each by a power of two to at most 2^15; the steps in
+                // turns between the warpgroups
+                for (int ch = t.q0 >> 2; ch <= (t.q1 - 1) >> 2; ch++) wait_ok(&bar.rfull[ch], nit & 1, ok);
+                unsigned char *Rm = Rs + (2 * w4) * (kChunkBytes / 8) + frow * 128;
+                float mx[2] = {0.f, 0.f};
+#pragma unroll 1
+                for (int st = t.q0 + (int)slot; st < t.q1; st += 2) {
+                    const unsigned char *base = Rm + (st >> 2) * kChunkBytes + (st & 3) * 1024;
+#pragma unroll
+                    for (int j = 0; j < 2; j++)
+#pragma unroll
+                        for (int h = 0; h < 2; h++) {
+                            const float4 x = *reinterpret_cast<const float4 *>(base + h * (kChunkBytes / 8) +
+                                                                               (fcol ^ (4 * j + frow)) * 16 + 512 * j);
+                            mx[h] = fmaxf(fmaxf(mx[h], finite_abs(x.x)), finite_abs(x.y));
+                            mx[h] = fmaxf(fmaxf(mx[h], finite_abs(x.z)), finite_abs(x.w));
+                        }
+                }
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 1));
+                    mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 2));
+                    if (frow == 0) kmax[slot][16 * w4 + 8 * h + fcol] = mx[h];
+                }
+                asm volatile("bar.sync 1, 256;" ::: "memory");
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int c = 16 * w4 + 8 * h + fcol;
+                    mx[h] = column_scale(fmaxf(kmax[0][c], kmax[1][c]));
+                }
+#pragma unroll 1
+                for (int st = t.q0 + (int)slot; st < t.q1; st += 2) {
+                    unsigned char *base = Rm + (st >> 2) * kChunkBytes + (st & 3) * 1024;
+#pragma unroll
+                    for (int j = 0; j < 2; j++)
+#pragma unroll
+                        for (int h = 0; h < 2; h++) {
+                            float4 &x = *reinterpret_cast<float4 *>(base + h * (kChunkBytes / 8) +
+                                                                    (fcol ^ (4 * j + frow)) * 16 + 512 * j);
+                            x = make_float4(x.x * mx[h], x.y * mx[h], x.z * mx[h], x.w * mx[h]);
+                        }
+                }
+                fence_proxy_async_smem();  // the scaled values before a later tile's loads over them
+                if (slot == 0) {
+                    if (nit >= 2) wait_ok(&bar.kfree[nit & 1], ((nit >> 1) - 1) & 1, ok);
+                    if (frow == 0) {
+                        kcol[nit & 1][16 * w4 + fcol] = mx[0];
+                        kcol[nit & 1][16 * w4 + 8 + fcol] = mx[1];
+                    }
+                }
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(&bar.rscaled);
+                    if (slot == 0) mbar_arrive(&bar.kfull[nit & 1]);
+                }
+                thr2[0] *= mx[0];
+                thr2[1] *= mx[1];
+            }
+            thr2[0] *= thr2[0];
+            thr2[1] *= thr2[1];
             for (int k = 0; k < nfy; k++) {
                 for (int i = 0; 2 * i < nb; i++, n++) {
                     if ((n & 1) != slot) {
@@ -562,7 +666,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                         tmem_zero16(u);
                         const int row = urow + 16 * (t.p0 + blk);
                         float2 a[2][2];
-                        float near = 3.402823466e38f;
+                        float near[2] = {3.402823466e38f, 3.402823466e38f};
 #pragma unroll
                         for (int j = 0; j < 2; j++)
 #pragma unroll
@@ -570,17 +674,18 @@ __global__ void __launch_bounds__(kThreads, 1)
                                 const float2 re = make_float2(r[h][4 * j], r[h][4 * j + 1]);
                                 const float2 im = make_float2(r[h][4 * j + 2], r[h][4 * j + 3]);
                                 a[j][h] = __ffma2_rn(im, im, __fmul2_rn(re, re));
-                                const float2 d = __fadd2_rn(a[j][h], make_float2(-thr2, -thr2));
-                                near = fminf(near, fminf(fabsf(d.x), fabsf(d.y)));
+                                const float2 d = __fadd2_rn(a[j][h], make_float2(-thr2[h], -thr2[h]));
+                                near[h] = fminf(near[h], fminf(fabsf(d.x), fabsf(d.y)));
                             }
-                        if (__any_sync(0xffffffffu, near < band)) {
+                        if (__any_sync(0xffffffffu, near[0] < kThrBand * thr2[0] || near[1] < kThrBand * thr2[1])) {
                             // what lies too near is decided in FP64, value by value
 #pragma unroll 1
                             for (int e = 0; e < 8; e++) {
                                 const int j = e >> 2, h = (e >> 1) & 1;
                                 const float2 v = j ? (h ? a[1][1] : a[1][0]) : (h ? a[0][1] : a[0][0]);
                                 const int y = row + 8 * j + (e & 1), x = t.x0 + 16 * w4 + 8 * h + fcol;
-                                const bool mine_ = fabsf((e & 1 ? v.y : v.x) - thr2) < band &&
+                                const float th = h ? thr2[1] : thr2[0];
+                                const bool mine_ = fabsf((e & 1 ? v.y : v.x) - th) < kThrBand * th &&
                                                    (unsigned)y < (unsigned)H && x < q.W;
                                 uint32_t todo = __ballot_sync(0xffffffffu, mine_);
                                 bool over = false;
@@ -607,7 +712,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                             for (int h = 0; h < 2; h++) {
                                 float2 re = make_float2(r[h][4 * j], r[h][4 * j + 1]);
                                 float2 im = make_float2(r[h][4 * j + 2], r[h][4 * j + 3]);
-                                const bool k0 = in0 && a[j][h].x >= thr2, k1 = in1 && a[j][h].y >= thr2;
+                                const bool k0 = in0 && a[j][h].x >= thr2[h], k1 = in1 && a[j][h].y >= thr2[h];
                                 re = make_float2(k0 ? re.x : 0.f, k1 ? re.y : 0.f);
                                 im = make_float2(k0 ? im.x : 0.f, k1 ? im.y : 0.f);
                                 split2(__fmul2_rn(re, ts), o[h][2 * j], o[h][4 + 2 * j]);
@@ -616,17 +721,20 @@ __global__ void __launch_bounds__(kThreads, 1)
                         }
                         __syncwarp();
                     };
-                    half(2 * i);
-                    if (mine > 0) wait_ok(&bar.a2free[slot], (mine - 1) & 1, ok);
-                    mine++;
-                    tc_fence_after();
-                    __syncwarp();
-                    tmem_st_16x128b_x4(a0, o[0]);
-                    tmem_st_16x128b_x4(a0 + (1u << 20), o[1]);
-                    if (2 * i + 1 < nb) {
-                        half(2 * i + 1);
-                        tmem_st_16x128b_x4(a0 + 16, o[0]);
-                        tmem_st_16x128b_x4(a0 + 16 + (1u << 20), o[1]);
+                    // one body for both halves: every SM sub-partition runs all roles, and their loops have to
+                    // fit the instruction cache together (a 1024^2 frame by the kernel's size in KB: 58 1.75 ms,
+                    // 71 1.79, 77 1.92, 84 2.17)
+#pragma unroll 1
+                    for (int hb = 0; hb < 2 && 2 * i + hb < nb; hb++) {
+                        half(2 * i + hb);
+                        if (hb == 0) {
+                            if (mine > 0) wait_ok(&bar.a2free[slot], (mine - 1) & 1, ok);
+                            mine++;
+                            tc_fence_after();
+                        }
+                        __syncwarp();
+                        tmem_st_16x128b_x4(a0 + 16 * hb, o[0]);
+                        tmem_st_16x128b_x4(a0 + 16 * hb + (1u << 20), o[1]);
                     }
                     tmem_wait_st();
                     tc_fence_before();
@@ -644,8 +752,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         // ---- C: modulate and sum the finished rows over wy; one block of each pair per warpgroup ----
         reg_inc<Cfg::RC>();
         const int par = wg - 5;
-        uint32_t nk = 0, parity = 0;
-        for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
+        uint32_t nk = 0, parity = 0, nit = 0;
+        for (int item = blockIdx.x; item < nitems; item += gridDim.x, nit++) {
             TcTile t;
             const TcSeq &q = tab.seq[tc_item<NS>(tab, nseq, item, list, listn, s, m, RW, t)];
             const int nfy = q.nfy, poff = ((t.y0 - t.ra) >> 1) + frow;
@@ -697,6 +805,15 @@ __global__ void __launch_bounds__(kThreads, 1)
                 parity ^= (1u << ((t.nc + 1) >> 1)) - 1;
             }
             const float mul = q.out_mul / *q.kr;
+            float inv[2] = {1.f, 1.f};  // of the columns' scales
+            if constexpr (!UNIT) {
+                const uint32_t b = nit & 1;
+                wait_ok(&bar.kfull[b], (nit >> 1) & 1, ok);
+                inv[0] = reciprocal_pow2(kcol[b][16 * w4 + fcol]);
+                inv[1] = reciprocal_pow2(kcol[b][16 * w4 + 8 + fcol]);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bar.kfree[b]);
+            }
             float2 *Cp = q.C + (size_t)t.plane * q.H * q.pitch + t.x0 + 16 * w4 + fcol;
 #pragma unroll
             for (int c = 0; c < RB; c++)
@@ -706,8 +823,10 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
                     for (int h = 0; h < 2; h++) {
                         const float2 re = are[c][h][j], im = aim[c][h][j];
-                        if (y < q.H) Cp[(size_t)y * q.pitch + 8 * h] = make_float2(re.x * mul, im.x * mul);
-                        if (y + 1 < q.H) Cp[(size_t)(y + 1) * q.pitch + 8 * h] = make_float2(re.y * mul, im.y * mul);
+                        if (y < q.H)
+                            Cp[(size_t)y * q.pitch + 8 * h] = make_float2(re.x * mul * inv[h], im.x * mul * inv[h]);
+                        if (y + 1 < q.H)
+                            Cp[(size_t)(y + 1) * q.pitch + 8 * h] = make_float2(re.y * mul * inv[h], im.y * mul * inv[h]);
                     }
                 }
         }
@@ -717,29 +836,6 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncthreads();
     tc_fence_after();
     if (warp == 0) tmem_dealloc(tmem, 512);
-}
-
-// max of |re| and |im| over the finite elements of f, as the bits of a float
-__global__ void __launch_bounds__(256) wff_absmax_kernel(const float2 *__restrict__ f, size_t n,
-                                                         uint32_t *__restrict__ out)
-{
-    float mx = 0.f;
-    for (size_t k = blockIdx.x * 256 + threadIdx.x; k < n; k += (size_t)gridDim.x * 256) {
-        const float2 v = f[k];
-        const float a = fabsf(v.x), b = fabsf(v.y);
-        if (a <= 3.402823466e38f) mx = fmaxf(mx, a);
-        if (b <= 3.402823466e38f) mx = fmaxf(mx, b);
-    }
-    const uint32_t w = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
-    if ((threadIdx.x & 31) == 0 && w) atomicMax(out, w);
-}
-
-// The power of two that R carries: with |f| <= max in each part, |R| stays below 2^15.
-__global__ void wff_tc_scale_kernel(const uint32_t *__restrict__ mx, float sum_gx, float *__restrict__ kr)
-{
-    const float b = __uint_as_float(*mx) * 1.4143f * sum_gx;
-    const int e = (int)((__float_as_uint(b) >> 23) & 255) - 126;  // b < 2^e
-    *kr = b > 0.f ? __uint_as_float((uint32_t)(127 + min(100, max(-100, 15 - e))) << 23) : 1.f;
 }
 
 // Tile heights (in pairs of blocks) whose accumulators fit the TMEM and whose
@@ -783,27 +879,35 @@ using Tc5 = TcCfg<5, 40, 48, 72, 112>;
 using Tc4 = TcCfg<4, 40, 56, 72, 104>;
 using Tc2 = TcCfg<2, 40, 64, 72, 88>;
 
-template <class Cfg, int NS>
+template <class Cfg, int NS, bool UNIT>
 int tc_launch(const TcTable<NS> &tab, int nseq, int nitems, int grid, const WffPlan &P, const int2 *list,
               const int *count, cudaStream_t s)
 {
-    GLSU_TRY(raise_smem_limit((const void *)wff_tc_kernel<Cfg, NS>, kSmem));
+    GLSU_TRY(raise_smem_limit((const void *)wff_tc_kernel<Cfg, NS, UNIT>, kSmem));
     const int N = (2 * P.sy + 16 + 15) / 16 * 16;
-    wff_tc_kernel<Cfg, NS><<<grid, kThreads, kSmem, s>>>(tab, nseq, nitems, P.sy, (P.sy + 3) / 4, N, P.tc_tscale,
-                                                        (const uint4 *)P.d_tctaps, P.d_err, list, count);
+    wff_tc_kernel<Cfg, NS, UNIT><<<grid, kThreads, kSmem, s>>>(tab, nseq, nitems, P.sy, (P.sy + 3) / 4, N,
+                                                              P.tc_tscale, (const uint4 *)P.d_tctaps, P.d_err, list,
+                                                              count);
     GLSU_CUDA_TRY(cudaGetLastError());
     return GLSU_OK;
 }
 
-template <int NS>
+template <int NS, bool UNIT>
 int tc_launch_rb(int rb, const TcTable<NS> &tab, int nseq, int nitems, int grid, const WffPlan &P, const int2 *list,
                  const int *count, cudaStream_t s)
 {
     switch (rb) {
-    case 5: return tc_launch<Tc5, NS>(tab, nseq, nitems, grid, P, list, count, s);
-    case 4: return tc_launch<Tc4, NS>(tab, nseq, nitems, grid, P, list, count, s);
-    default: return tc_launch<Tc2, NS>(tab, nseq, nitems, grid, P, list, count, s);
+    case 5: return tc_launch<Tc5, NS, UNIT>(tab, nseq, nitems, grid, P, list, count, s);
+    case 4: return tc_launch<Tc4, NS, UNIT>(tab, nseq, nitems, grid, P, list, count, s);
+    default: return tc_launch<Tc2, NS, UNIT>(tab, nseq, nitems, grid, P, list, count, s);
     }
+}
+
+int tc_launch_one(int rb, const TcTable<1> &tab, int nitems, int grid, const WffPlan &P, const int2 *list,
+                  const int *count, cudaStream_t s)
+{
+    return P.unit_input ? tc_launch_rb<1, true>(rb, tab, 1, nitems, grid, P, list, count, s)
+                        : tc_launch_rb<1, false>(rb, tab, 1, nitems, grid, P, list, count, s);
 }
 
 void tc_seq(TcSeq &q, const WffPlan &P, int rw, int item0)
@@ -860,7 +964,6 @@ int WffPlan::init_tc()
         }
     // T = tscale U stays below 2^15 as R does
     tc_tscale = (float)std::ldexp(1.0, -(kTapShift + std::max(0, (int)std::ceil(std::log2(sum)))));
-    tc_sum_gx = (float)sumx;
     std::vector<float> ey((size_t)nfy * eys2 * 4);
     for (int k = 0; k < nfy; k++) {
         const double wy = p.wyl + (double)k * p.wyi;
@@ -872,13 +975,13 @@ int WffPlan::init_tc()
             }
     }
     if (cudaMalloc(&d_tctaps, tb.size() * 2) != cudaSuccess || cudaMalloc(&d_ey2, ey.size() * 4) != cudaSuccess ||
-        cudaMalloc(&d_kr, 2 * sizeof(float)) != cudaSuccess)
+        cudaMalloc(&d_kr, sizeof(float)) != cudaSuccess)
         return fail(GLSU_ERR_ALLOC, "cudaMalloc of the tensor-core sweep's tables failed");
     GLSU_CUDA_TRY(cudaMemcpy(d_tctaps, tb.data(), tb.size() * 2, cudaMemcpyHostToDevice));
     GLSU_CUDA_TRY(cudaMemcpy(d_ey2, ey.data(), ey.size() * 4, cudaMemcpyHostToDevice));
-    // scale of an input of unit modulus (DPRA); other inputs get theirs per call
-    const float kr[2] = {(float)std::ldexp(1.0, 15 - std::ilogb((float)(1.4143f * sumx)) - 1), 0.f};
-    GLSU_CUDA_TRY(cudaMemcpy(d_kr, kr, sizeof(kr), cudaMemcpyHostToDevice));
+    // an input of unit modulus (DPRA) is scaled by the row pass, others by column and tile in the sweep
+    const float kr = unit_input ? (float)std::ldexp(1.0, 15 - std::ilogb((float)(1.4143f * sumx)) - 1) : 1.f;
+    GLSU_CUDA_TRY(cudaMemcpy(d_kr, &kr, sizeof(kr), cudaMemcpyHostToDevice));
     auto enc = get_encode_fn();
     if (!enc) return fail(GLSU_ERR_CUDA, "cuTensorMapEncodeTiled unavailable");
     const cuuint64_t pairs = (cuuint64_t)(H + 1) / 2;
@@ -899,19 +1002,6 @@ void WffPlan::release_tc()
     cudaFree(d_kr);
     d_tctaps = d_ey2 = nullptr;
     d_kr = nullptr;
-}
-
-// Scale of R for this input (d_kr[0]); d_kr[1] holds the running maximum.
-int launch_tc_scale(const WffPlan &P, const void *d_f, cudaStream_t s)
-{
-    uint32_t *mx = (uint32_t *)P.d_kr + 1;
-    GLSU_CUDA_TRY(cudaMemsetAsync(mx, 0, sizeof(uint32_t), s));
-    const size_t n = (size_t)P.W * P.H;
-    wff_absmax_kernel<<<(int)std::min<size_t>((n + 1023) / 1024, 4 * (size_t)device_sm_count()), 256, 0, s>>>(
-        (const float2 *)d_f, n, mx);
-    wff_tc_scale_kernel<<<1, 1, 0, s>>>(mx, P.tc_sum_gx, P.d_kr);
-    GLSU_CUDA_TRY(cudaGetLastError());
-    return GLSU_OK;
 }
 
 // Modelled time (ms): the steps of the busiest SM at 250 cycles each (measured
@@ -949,7 +1039,7 @@ int launch_tc_sweep(const WffPlan *const *plans, int n, cudaStream_t s)
         const int tiles = tab.seq[0].ncg * tab.seq[0].nty;
         if (!P.mask.flags) {
             const int items = tiles * P.nfx;
-            return tc_launch_rb<1>(rb, tab, 1, items, std::min(items, sms), P, nullptr, nullptr, s);
+            return tc_launch_one(rb, tab, items, std::min(items, sms), P, nullptr, nullptr, s);
         }
         // tile-masked run: the tiles whose outputs, grown by sx columns, meet a
         // flagged tile.  A tile's results depend on its own rows of R only, and
@@ -959,7 +1049,7 @@ int launch_tc_sweep(const WffPlan *const *plans, int n, cudaStream_t s)
         mk.my = 0;
         mk.mx = P.sx;
         GLSU_TRY(launch_mask_list(mk, tab.seq[0].ncg, tab.seq[0].nty, 32 * rb, kCols, P.d_list, P.d_list_count, s));
-        return tc_launch_rb<1>(rb, tab, 1, P.nfx, std::min(tiles * P.nfx, sms), P, P.d_list, P.d_list_count, s);
+        return tc_launch_one(rb, tab, P.nfx, std::min(tiles * P.nfx, sms), P, P.d_list, P.d_list_count, s);
     }
     constexpr int NS = 64;
     static thread_local TcTable<NS> tab;
@@ -968,12 +1058,13 @@ int launch_tc_sweep(const WffPlan *const *plans, int n, cudaStream_t s)
         int items = 0;
         for (int k = 0; k < c; k++) {
             const WffPlan &P = *plans[i0 + k];
-            if (P.sy != plans[0]->sy || P.p.sigma_y != plans[0]->p.sigma_y || P.mask.flags || !P.use_tc())
-                return fail(GLSU_ERR_INVALID, "batched column sweep: plans of one window only");
+            if (P.sy != plans[0]->sy || P.p.sigma_y != plans[0]->p.sigma_y || P.mask.flags || !P.use_tc() ||
+                !P.unit_input)
+                return fail(GLSU_ERR_INVALID, "batched column sweep: plans of one window and unit modulus only");
             tc_seq(tab.seq[k], P, 32 * rb, items);
             items += tab.seq[k].ncg * tab.seq[k].nty * P.nfx;
         }
-        GLSU_TRY(tc_launch_rb<NS>(rb, tab, c, items, std::min(items, sms), *plans[i0], nullptr, nullptr, s));
+        GLSU_TRY((tc_launch_rb<NS, true>(rb, tab, c, items, std::min(items, sms), *plans[i0], nullptr, nullptr, s)));
     }
     return GLSU_OK;
 }

@@ -146,3 +146,23 @@ def test_one_pair_of_blocks_a_wy(glsu, oracle, shape, sigma):
     ref, _ = oracle.wff2(f.astype(np.complex128), *p.tuple())
     assert np.array_equal(outs[0], outs[1]) and np.array_equal(outs[0], outs[2])
     assert np.abs(outs[0] - ref).max() <= TOL * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("size", [1e5, 1e9, 1e30])
+def test_a_large_finite_pixel_stays_in_its_columns_and_tiles(glsu, size):
+    """Columns beyond both row filters' reach of one large pixel (as for a
+    non-finite one), and rows of tiles that do not read it (a tile is at most 160
+    rows and reads 2s + 16 more on either side), have the bits they have without
+    it.  In the rows of its own tiles and columns that no filter connects with it
+    (2s away), R is off by 2^-25 of a value scaled to 2^15: 2^-40 of the pixel."""
+    f = _field((700, 200), 8)
+    f[50, 30] = 0
+    a, _ = _run(glsu, f, 5.0, sigx=4.0)
+    f[50, 30] = size
+    b, _ = _run(glsu, f, 5.0, sigx=4.0)
+    far = 30 + 2 * 12 + 1
+    assert np.array_equal(a[:, far:], b[:, far:])
+    assert np.array_equal(a[320:], b[320:])
+    if size == 1e5:
+        top = np.abs(a).max()
+        assert np.abs(a - b)[50 + 2 * 15 + 1:].max() <= TOL * top
