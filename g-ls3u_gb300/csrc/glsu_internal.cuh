@@ -210,6 +210,8 @@ struct WffPlan {
     int autotune(cudaStream_t s);
     int choose_by_model();
     double model_ms(int method) const;
+    double colfft_model_ms() const;
+    bool local_sweep() const;
     int column_method() const
     {
         return (method == GLSU_METHOD_AUTO || method == GLSU_METHOD_TIMED) ? auto_method : method;
@@ -224,6 +226,8 @@ struct WffPlan {
     void *d_tctaps = nullptr;  // B operand of the banded products, hi and lo FP16 parts
     void *d_ey2 = nullptr;     // wy phasors of row pairs
     float *d_kr = nullptr;     // the power of two that R carries
+    bool tc_local = false;     // wide columns are done again directly (AUTO, in the direct kernel's place)
+    uint8_t *d_tcwide = nullptr;
     CUtensorMap tmT;           // d_R in row pairs: {4 pitch floats, (H + 1) / 2, nfx}
     float tc_tscale = 1;
     bool tc_supported() const;

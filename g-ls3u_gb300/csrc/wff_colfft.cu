@@ -278,18 +278,30 @@ constexpr double kModelLaunchMs = 0.05;
 // over the 2S-row halo of each 128-row tile, at a rate per instantiation.
 // FFT sweep: per column and x-frequency, 2 nfy + 2 transforms of length L
 // in a number of radix passes.
+double WffPlan::colfft_model_ms() const
+{
+    const double units = (double)pitch * nfx * fft_L * (fft_nst * (2.0 * nfy + 2.0) + kModelFftColumnUnits);
+    return units / kModelFftRate * 1e3 + kModelLaunchMs;
+}
+
 double WffPlan::model_ms(int m) const
 {
     if (m == GLSU_METHOD_FFT) {
         if (fft_L == 0) return 1e30;
-        if (d_tctaps) return tc_model_ms(*this);
-        const double units = (double)pitch * nfx * fft_L * (fft_nst * (2.0 * nfy + 2.0) + kModelFftColumnUnits);
-        return units / kModelFftRate * 1e3 + kModelLaunchMs;
+        return d_tctaps ? tc_model_ms(*this) : colfft_model_ms();
     }
     const int S = syi;
     const double taps = (2.0 * S + 1.0) * (2.0 + 2.0 * S / 128.0);
     const double rate = S <= 30 ? kModelDirectRate30 : (S <= 45 ? kModelDirectRate45 : kModelDirectRate60);
     return (double)pitch * H * nfx * nfy * taps / rate * 1e3 + kModelLaunchMs;
+}
+
+// Whether the direct kernel would be taken before the FFT sweep: the tensor-core
+// sweep in its place then keeps the reach it has (a value acts on 2s rows), which
+// the FFT sweep does not have either.
+bool WffPlan::local_sweep() const
+{
+    return !unit_input && d_tctaps && colfft_model_ms() >= 0.9 * model_ms(GLSU_METHOD_DIRECT);
 }
 
 // AUTO without timing: the shortest compiled transform length (built by
@@ -305,6 +317,7 @@ int WffPlan::choose_by_model()
     tune_ms_direct = (float)model_ms(GLSU_METHOD_DIRECT);
     tune_ms_fft = (float)model_ms(GLSU_METHOD_FFT);
     if (tune_ms_fft < 0.9f * tune_ms_direct) auto_method = GLSU_METHOD_FFT;
+    tc_local = local_sweep();
     return ensure_colfft();
 }
 
@@ -390,6 +403,7 @@ int WffPlan::autotune(cudaStream_t s)
     tune_ms_fft = r.ms_fft;
     if (r.L != fft_L) GLSU_TRY(set_fft_len(r.L));
     fft_explicit = !r.tc;
+    tc_local = local_sweep();
     GLSU_TRY(set_fft_plan(r.nc, r.order));
     return ensure_colfft();
 }

@@ -19,7 +19,8 @@
 // 2^15.  An input of unit modulus (DPRA) has one scale, which the row pass
 // applies (d_kr); for any other the B warps scale each column of a tile by its
 // own largest finite value, so that a large value leaves its mark, 2^-40 of
-// itself, on its own columns and tiles only.
+// itself, on its own columns and tiles only.  (Where the direct kernel's shorter
+// reach is to be kept, wff_tc_local_kernel does such columns of a tile again.)
 //
 // One CTA of seven warpgroups per SM walks a list of (plane, 64 columns, Rw
 // rows) tiles; the tile of R (Rw + 4s rows) stays in shared memory for all
@@ -58,6 +59,7 @@
 
 #include "glsu_internal.cuh"
 #include "ptx_sm103.cuh"
+#include "wff_common.cuh"
 
 namespace glsu {
 namespace {
@@ -83,7 +85,7 @@ constexpr int kTapShift = 6;                // taps scaled by 2^6
 // the error against 64 bits at sigma 10 goes from 5.9e-7 to 1.4e-7 of the
 // output's norm, that of the FFT sweep.
 constexpr double kShrink = 0.82e-8;
-constexpr int kScaleBytes = 4 * kCols * 4;  // column scales of two tiles, column maxima by two warpgroups
+constexpr int kScaleBytes = 6 * kCols * 4;  // column scales of two tiles; column maxima and smallest block maxima
 constexpr int kSmem = kMaxChunks * kChunkBytes + kPhRing * kPhBytes + kMaxTapBytes + 768 + kScaleBytes + 1024;
 static_assert(kSmem <= 227 * 1024, "column tile exceeds shared memory");
 
@@ -94,6 +96,7 @@ struct TcSeq {
     float2 *C;
     const float *thr;
     const float *kr;     // scale that R carries
+    uint8_t *wide;       // per tile and column: its values' range is wide (nullptr: not asked for)
     const float *R;      // the planes that tm maps, [plane][row pair][pitch](re, re', im, im')
     double thr_exact;    // thr_mul without what the accumulation's truncation takes
     int H, W, pitch, nfy, eys2, ncg, nty, item0;
@@ -214,6 +217,10 @@ __device__ __forceinline__ float finite_abs(float v)
     const float a = fabsf(v);
     return a <= 3.402823466e38f ? a : 0.f;
 }
+// A column of a tile is wide where its largest value passes that of one of its
+// 16-row blocks by more: what the parts drop (2^-40 of the largest) is then more than
+// 2^-24 of that block.  Wide too is one with a value that is not finite.
+constexpr float kWide = 65536.f;
 // The power of two by which a column of R whose parts' largest magnitude is mx is multiplied: its
 // values times a phasor then stay below 2^15.
 __device__ __forceinline__ float column_scale(float mx)
@@ -353,7 +360,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     unsigned char *tb = reinterpret_cast<unsigned char *>(ph + kPhRing * kPhPairs);
     TcBars &bar = *reinterpret_cast<TcBars *>(tb + kMaxTapBytes);
     float(*kcol)[kCols] = reinterpret_cast<float(*)[kCols]>(tb + kMaxTapBytes + 768);  // of two tiles, in turns
-    float(*kmax)[kCols] = kcol + 2;
+    float(*kmax)[kCols] = kcol + 2, (*kmin)[kCols] = kcol + 4;  // by the two warpgroups that scale
 
     // warp-uniform to the compiler too: the operands of the tcgen05 instructions derive from it
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31, wg = warp >> 2, w4 = warp & 3;
@@ -583,9 +590,10 @@ __global__ void __launch_bounds__(kThreads, 1)
                 // turns between the warpgroups
                 for (int ch = t.q0 >> 2; ch <= (t.q1 - 1) >> 2; ch++) wait_ok(&bar.rfull[ch], nit & 1, ok);
                 unsigned char *Rm = Rs + (2 * w4) * (kChunkBytes / 8) + frow * 128;
-                float mx[2] = {0.f, 0.f};
+                float mx[2] = {0.f, 0.f}, mn[2] = {3.402823466e38f, 3.402823466e38f};
 #pragma unroll 1
                 for (int st = t.q0 + (int)slot; st < t.q1; st += 2) {
+                    float bm[2] = {0.f, 0.f};  // of the step's 16 rows
                     const unsigned char *base = Rm + (st >> 2) * kChunkBytes + (st & 3) * 1024;
 #pragma unroll
                     for (int j = 0; j < 2; j++)
@@ -593,21 +601,35 @@ __global__ void __launch_bounds__(kThreads, 1)
                         for (int h = 0; h < 2; h++) {
                             const float4 x = *reinterpret_cast<const float4 *>(base + h * (kChunkBytes / 8) +
                                                                                (fcol ^ (4 * j + frow)) * 16 + 512 * j);
-                            mx[h] = fmaxf(fmaxf(mx[h], finite_abs(x.x)), finite_abs(x.y));
-                            mx[h] = fmaxf(fmaxf(mx[h], finite_abs(x.z)), finite_abs(x.w));
+                            bm[h] = fmaxf(fmaxf(bm[h], finite_abs(x.x)), finite_abs(x.y));
+                            bm[h] = fmaxf(fmaxf(bm[h], finite_abs(x.z)), finite_abs(x.w));
+                            if (!(isfinite(x.x) && isfinite(x.y) && isfinite(x.z) && isfinite(x.w))) mn[h] = 0.f;
                         }
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        bm[h] = fmaxf(bm[h], __shfl_xor_sync(0xffffffffu, bm[h], 1));
+                        bm[h] = fmaxf(bm[h], __shfl_xor_sync(0xffffffffu, bm[h], 2));
+                        mx[h] = fmaxf(mx[h], bm[h]);
+                        if (bm[h] > 0.f) mn[h] = fminf(mn[h], bm[h]);
+                    }
                 }
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
-                    mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 1));
-                    mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 2));
-                    if (frow == 0) kmax[slot][16 * w4 + 8 * h + fcol] = mx[h];
+                    mn[h] = fminf(mn[h], __shfl_xor_sync(0xffffffffu, mn[h], 1));
+                    mn[h] = fminf(mn[h], __shfl_xor_sync(0xffffffffu, mn[h], 2));
+                    if (frow == 0) {
+                        kmax[slot][16 * w4 + 8 * h + fcol] = mx[h];
+                        kmin[slot][16 * w4 + 8 * h + fcol] = mn[h];
+                    }
                 }
                 asm volatile("bar.sync 1, 256;" ::: "memory");
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
                     const int c = 16 * w4 + 8 * h + fcol;
-                    mx[h] = column_scale(fmaxf(kmax[0][c], kmax[1][c]));
+                    const float top = fmaxf(kmax[0][c], kmax[1][c]);
+                    if (q.wide && slot == 0 && frow == 0)
+                        q.wide[(size_t)item * kCols + c] = top > kWide * fminf(kmin[0][c], kmin[1][c]);
+                    mx[h] = column_scale(top);
                 }
 #pragma unroll 1
                 for (int st = t.q0 + (int)slot; st < t.q1; st += 2) {
@@ -838,6 +860,81 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (warp == 0) tmem_dealloc(tmem, 512);
 }
 
+// The wide columns of a tile once more, directly in FP32 from R, as the direct
+// column kernel does them: a value then acts on the 2s rows around it only.  Runs
+// where AUTO would take the direct kernel but for this file (WffPlan::tc_local) and
+// the input is not of unit modulus.  One CTA a tile; with no wide column, the rule on
+// measured fields, it costs its launch.
+constexpr int kLocalThreads = 256;
+__global__ void __launch_bounds__(kLocalThreads) wff_tc_local_kernel(const __grid_constant__ TcTable<1> tab, int nitems,
+                                                                     int s, int m, int rw,
+                                                                     const __grid_constant__ Taps<float, 60> gA,
+                                                                     const __grid_constant__ Taps<float, 60> gB)
+{
+    __shared__ float2 D[kMaxChunks * kChunkRows], T[kMaxChunks * kChunkRows];
+    __shared__ float a[2 * kMaxTcHalf + 1], b[2 * kMaxTcHalf + 1];
+    __shared__ uint8_t wide[kCols];
+    const TcSeq &q = tab.seq[0];
+    const int tid = threadIdx.x;
+    for (int j = tid; j <= 2 * s; j += kLocalThreads) {
+        a[j] = gA.g[60 - s + j];
+        b[j] = gB.g[60 - s + j];
+    }
+    const float thr = *q.thr, thr2 = thr * thr;
+    const int pairs = (q.H + 1) >> 1;
+    for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
+        __syncthreads();
+        if (tid < kCols) wide[tid] = q.wide[(size_t)item * kCols + tid];
+        if (!__syncthreads_or(tid < kCols && wide[tid])) continue;
+        TcTile t;
+        tc_item<1>(tab, 1, item, nullptr, 0, s, m, rw, t);
+        const int y1 = min(t.y0 + rw, q.H), nu = y1 - t.y0 + 2 * s, nr = nu + 2 * s;
+        for (int c = 0; c < kCols && t.x0 + c < q.W; c++) {
+            if (!wide[c]) continue;
+            const float *R = q.R + ((size_t)t.plane * pairs * q.pitch + t.x0 + c) * 4;
+            float2 acc = make_float2(0.f, 0.f);  // of row t.y0 + tid: rw <= kLocalThreads
+            for (int k = 0; k < q.nfy; k++) {
+                const float *P = reinterpret_cast<const float *>(q.ey2 + (size_t)k * q.eys2 + kTcPad);
+                for (int i = tid; i < nr; i += kLocalThreads) {
+                    const int y = t.y0 - 2 * s + i;
+                    float2 d = make_float2(0.f, 0.f);
+                    if ((unsigned)y < (unsigned)q.H) {
+                        const float *e = R + (size_t)(y >> 1) * q.pitch * 4 + (y & 1), *p = P + (y >> 1) * 4 + (y & 1);
+                        d = make_float2(e[0] * p[0] - e[2] * p[2], e[0] * p[2] + e[2] * p[0]);
+                    }
+                    D[i] = d;
+                }
+                __syncthreads();
+                for (int i = tid; i < nu; i += kLocalThreads) {
+                    const int y = t.y0 - s + i;
+                    float2 u = make_float2(0.f, 0.f);
+                    for (int j = 0; j <= 2 * s; j++) {
+                        u.x = fmaf(a[j], D[i + j].x, u.x);
+                        u.y = fmaf(a[j], D[i + j].y, u.y);
+                    }
+                    const bool keep = (unsigned)y < (unsigned)q.H && u.x * u.x + u.y * u.y >= thr2;
+                    T[i] = keep ? u : make_float2(0.f, 0.f);
+                }
+                __syncthreads();
+                if (t.y0 + tid < y1) {
+                    const int y = t.y0 + tid;
+                    float2 v = make_float2(0.f, 0.f);
+                    for (int j = 0; j <= 2 * s; j++) {
+                        v.x = fmaf(b[j], T[tid + j].x, v.x);
+                        v.y = fmaf(b[j], T[tid + j].y, v.y);
+                    }
+                    const float *p = P + (y >> 1) * 4 + (y & 1);
+                    acc.x += p[0] * v.x + p[2] * v.y;
+                    acc.y += p[0] * v.y - p[2] * v.x;
+                }
+            }
+            __syncthreads();
+            if (t.y0 + tid < y1)
+                q.C[(size_t)t.plane * q.H * q.pitch + (size_t)(t.y0 + tid) * q.pitch + t.x0 + c] = acc;
+        }
+    }
+}
+
 // Tile heights (in pairs of blocks) whose accumulators fit the TMEM and whose
 // rows of R fit the shared memory at half-size s, largest first.
 int tc_row_blocks(int s, int *rb)
@@ -917,6 +1014,7 @@ void tc_seq(TcSeq &q, const WffPlan &P, int rw, int item0)
     q.C = (float2 *)P.d_C;
     q.thr = (const float *)P.d_thr;
     q.kr = (const float *)P.d_kr;
+    q.wide = P.tc_local ? P.d_tcwide : nullptr;
     q.R = (const float *)P.d_R;
     q.H = P.H;
     q.W = P.W;
@@ -975,7 +1073,9 @@ int WffPlan::init_tc()
             }
     }
     if (cudaMalloc(&d_tctaps, tb.size() * 2) != cudaSuccess || cudaMalloc(&d_ey2, ey.size() * 4) != cudaSuccess ||
-        cudaMalloc(&d_kr, sizeof(float)) != cudaSuccess)
+        cudaMalloc(&d_kr, sizeof(float)) != cudaSuccess ||
+        (!unit_input && cudaMalloc(&d_tcwide, (size_t)nfx * ((H + 63) / 64) * ((W + kCols - 1) / kCols) * kCols) !=
+                            cudaSuccess))
         return fail(GLSU_ERR_ALLOC, "cudaMalloc of the tensor-core sweep's tables failed");
     GLSU_CUDA_TRY(cudaMemcpy(d_tctaps, tb.data(), tb.size() * 2, cudaMemcpyHostToDevice));
     GLSU_CUDA_TRY(cudaMemcpy(d_ey2, ey.data(), ey.size() * 4, cudaMemcpyHostToDevice));
@@ -1000,7 +1100,9 @@ void WffPlan::release_tc()
     cudaFree(d_tctaps);
     cudaFree(d_ey2);
     cudaFree(d_kr);
+    cudaFree(d_tcwide);
     d_tctaps = d_ey2 = nullptr;
+    d_tcwide = nullptr;
     d_kr = nullptr;
 }
 
@@ -1039,12 +1141,19 @@ int launch_tc_sweep(const WffPlan *const *plans, int n, cudaStream_t s)
         const int tiles = tab.seq[0].ncg * tab.seq[0].nty;
         if (!P.mask.flags) {
             const int items = tiles * P.nfx;
-            return tc_launch_one(rb, tab, items, std::min(items, sms), P, nullptr, nullptr, s);
+            GLSU_TRY(tc_launch_one(rb, tab, items, std::min(items, sms), P, nullptr, nullptr, s));
+            if (!tab.seq[0].wide) return GLSU_OK;
+            wff_tc_local_kernel<<<std::min(items, 2 * sms), kLocalThreads, 0, s>>>(
+                tab, items, P.sy, (P.sy + 3) / 4, 32 * rb, make_taps<float, 60>(P.gy, P.sy, P.inv_norm),
+                make_taps<float, 60>(P.gy, P.sy, 1.0));
+            GLSU_CUDA_TRY(cudaGetLastError());
+            return GLSU_OK;
         }
         // tile-masked run: the tiles whose outputs, grown by sx columns, meet a
         // flagged tile.  A tile's results depend on its own rows of R only, and
         // ring positions on image rows, so they are the full frame's bits.
         if (!P.d_list) return fail(GLSU_ERR_INVALID, "tile-masked run without a tile list buffer");
+        tab.seq[0].wide = nullptr;
         TileMask mk = P.mask;
         mk.my = 0;
         mk.mx = P.sx;

@@ -166,3 +166,52 @@ def test_a_large_finite_pixel_stays_in_its_columns_and_tiles(glsu, size):
     if size == 1e5:
         top = np.abs(a).max()
         assert np.abs(a - b)[50 + 2 * 15 + 1:].max() <= TOL * top
+
+
+@pytest.mark.parametrize("bad", [1e9, 1e30, np.inf, np.nan])
+def test_auto_keeps_the_direct_kernels_reach(glsu, bad):
+    """With a window for which AUTO would take the direct kernel before the FFT
+    sweep, one pixel acts on the rows that two column filters connect with it (40, as
+    the direct kernel is compiled for half-size 20) and on no others."""
+    import torch
+    f = _field((500, 200), 10)
+    p = glsu.WffParams(4.0, -0.4, 0.4, 0.05, 5.0, -0.4, 0.4, 0.05, 0.0)
+
+    def run(v, direct):
+        g = f.copy()
+        g[250, 60] = v
+        t = torch.from_numpy(g).cuda()
+        out = torch.empty_like(t)
+        w = glsu.WFF2(200, 500, "f32", p)
+        assert w.tuning()["method"] == glsu.METHOD_FFT
+        if direct:
+            w.set_method(glsu.METHOD_DIRECT)
+        w.run(t.data_ptr(), out.data_ptr())
+        w.close()
+        return out.cpu().numpy()
+
+    a, b, d = run(0, False), run(bad, False), run(bad, True)
+    far = np.r_[0:250 - 40, 250 + 41:500]
+    assert np.abs(a - b)[far].max() <= TOL * np.abs(a).max()
+    assert np.abs(d - b)[far].max() <= TOL * np.abs(a).max()
+    if np.isfinite(bad):
+        assert np.abs(d - b).max() <= TOL * np.abs(d).max()
+
+
+def test_wide_columns_over_many_tiles(glsu, oracle):
+    """A field whose amplitude falls by 2^20 within every tile, odd sizes: every
+    column is done directly; the FP32 form's bar by rows of like size."""
+    import torch
+    y, x = np.mgrid[0:333, 0:200].astype(np.float64)
+    amp = np.exp2(-20.0 * np.abs(((y + 20) % 64) / 32 - 1))
+    f = (amp * np.exp(1j * (0.2 * x - 0.1 * y))).astype(np.complex64)
+    p = glsu.WffParams(2.0, -0.4, 0.4, 0.05, 2.0, -0.4, 0.4, 0.05, 0.0)
+    t = torch.from_numpy(f).cuda()
+    out = torch.empty_like(t)
+    w = glsu.WFF2(200, 333, "f32", p)
+    assert w.tuning()["method"] == glsu.METHOD_FFT
+    w.run(t.data_ptr(), out.data_ptr())
+    w.close()
+    ref, _ = oracle.wff2(f.astype(np.complex128), *p.tuple())
+    err = np.abs(out.cpu().numpy() - ref).max(1)
+    assert (err <= TOL * np.abs(ref).max(1)).all()
