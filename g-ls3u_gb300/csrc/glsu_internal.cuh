@@ -230,6 +230,7 @@ struct WffPlan {
     uint8_t *d_tcwide = nullptr;
     CUtensorMap tmT;           // d_R in row pairs: {4 pitch floats, (H + 1) / 2, nfx}
     float tc_tscale = 1;
+    double tc_shrink = 0;      // what the accumulation's truncation takes of a pass
     bool tc_supported() const;
     int init_tc();
     void release_tc();

@@ -215,3 +215,40 @@ def test_wide_columns_over_many_tiles(glsu, oracle):
     ref, _ = oracle.wff2(f.astype(np.complex128), *p.tuple())
     err = np.abs(out.cpu().numpy() - ref).max(1)
     assert (err <= TOL * np.abs(ref).max(1)).all()
+
+
+@pytest.mark.parametrize("kind", ["constant", "wave", "noise"])
+@pytest.mark.parametrize("half", [15, 30, 45])
+def test_error_and_scale_of_a_single_frequency(glsu, oracle, half, kind):
+    """The sums' truncation is balanced and its mean taken out.  Uncorrected, the
+    output is 2.3, 3.8 and 6.4e-7 too small at these half-sizes (twice a pass's
+    loss), and a constant column, whose low parts would all have one sign, is off by
+    up to 6e-7 beside that.  Bars of the output's norm: its scale within 2e-7 (0.4e-7
+    a pass between kinds of data, and as much for the FP32 row filters), the error
+    within 4e-7 (a pass: 3 x 16 products for each of at most 7 steps cut off by up
+    to 2^-26, and 21 sums by up to 2^-23, at random: 2.2e-7; twice, and the filters)."""
+    import torch
+    rng = np.random.default_rng(half)
+    H, W = 320, 96
+    y = np.arange(H)[:, None]
+    amp = np.exp2(rng.uniform(-1, 0, W))[None]
+    phase = rng.uniform(0, 2 * np.pi, W)[None]
+    if kind == "constant":
+        f = amp * np.exp(1j * (phase + 0 * y))
+    elif kind == "wave":
+        f = amp * np.exp(1j * (phase + 0.02 * y + 2 * np.cos(y / 40.0)))
+    else:
+        f = rng.standard_normal((H, W)) + 1j * rng.standard_normal((H, W))
+    f = f.astype(np.complex64)
+    p = glsu.WffParams(0.1, 0.0, 0.0, 1.0, half / 3.0, 0.0, 0.0, 1.0, 0.0)
+    t = torch.from_numpy(f).cuda()
+    out = torch.empty_like(t)
+    w = glsu.WFF2(W, H, "f32", p)
+    w.set_method(glsu.METHOD_FFT)
+    w.run(t.data_ptr(), out.data_ptr())
+    w.close()
+    out = out.cpu().numpy().astype(np.complex128)
+    ref, _ = oracle.wff2(f.astype(np.complex128), *p.tuple())
+    power = (np.abs(ref) ** 2).sum()
+    assert abs((np.conj(ref) * (out - ref)).sum().real / power) <= 2e-7
+    assert np.sqrt((np.abs(out - ref) ** 2).sum() / power) <= 4e-7
