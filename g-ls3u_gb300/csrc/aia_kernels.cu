@@ -204,15 +204,18 @@ __global__ void __launch_bounds__(kAiaThreads)
     __shared__ AiaTables T;
     __shared__ ff red[kAiaThreads / 32][5 + 3 * MM];
     __shared__ bool last;
+    __shared__ ff d0;  // FINAL: delta_0 in [-pi, pi]; the shifts given by a caller may be any
     const int tid = threadIdx.x;
+    if (FINAL && tid == 0) {
+        double sn, cs;
+        sincos(state[0], &sn, &cs);
+        d0 = ff_of(atan2(sn, cs));
+    }
     for (int e = tid; e < (int)(sizeof(AiaTables) / 4); e += kAiaThreads)
         reinterpret_cast<float *>(&T)[e] = __ldcg(reinterpret_cast<const float *>(tab) + e);
     __syncthreads();
     ff acc[FINAL ? 1 : 5 + 3 * MM];
-    ff d0 = {0.f, 0.f};
-    if constexpr (FINAL) {
-        d0 = ff_of(state[0]);
-    } else {
+    if constexpr (!FINAL) {
 #pragma unroll
         for (int v = 0; v < 5 + 3 * MM; v++) acc[v] = ff{0.f, 0.f};
     }
