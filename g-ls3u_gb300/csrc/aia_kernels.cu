@@ -84,8 +84,9 @@ __device__ void aia_tables(const double *__restrict__ state, int M, double *cs, 
     }
 }
 
-// (X, -Y) / hypot(X, Y) in float-float; (1, 0) where both vanish.
-__device__ __forceinline__ void aia_unit(ff X, ff Y, ff *c, ff *s)
+// (X, -Y) / hypot(X, Y) in float-float; (1, 0) where both vanish.  False where
+// that is not finite, with no number in *c and *s.
+__device__ __forceinline__ bool aia_unit(ff X, ff Y, ff *c, ff *s)
 {
     // scaled by a power of two so that the larger part is in [1, 2)
     const float mx = fmaxf(fabsf(X.hi), fabsf(Y.hi));
@@ -94,10 +95,10 @@ __device__ __forceinline__ void aia_unit(ff X, ff Y, ff *c, ff *s)
     X = ff{X.hi * sc, X.lo * sc};
     Y = ff{Y.hi * sc, Y.lo * sc};
     const float n = fmaf(X.hi, X.hi, Y.hi * Y.hi);
-    if (!(n > 0.f)) {
-        *c = ff{1.f, 0.f};
-        *s = ff{0.f, 0.f};
-        return;
+    if (!(n > 0.f && n <= 3.402823466e38f)) {
+        *c = ff{n == 0.f ? 1.f : n - n, 0.f};
+        *s = ff{n == 0.f ? 0.f : n - n, 0.f};
+        return n == 0.f;
     }
     const float r = rsqrtf(n);
     const ff u = ff_mul_f(X, r), v = ff_mul_f(Y, r);  // within 2^-22 of unit length
@@ -106,6 +107,7 @@ __device__ __forceinline__ void aia_unit(ff X, ff Y, ff *c, ff *s)
     const float k = d * fmaf(0.375f, d, 0.5f);        // (1 - d)^(-1/2) - 1
     *c = ff_fast_two_sum(u.hi, fmaf(u.hi, k, u.lo));
     *s = ff_neg(ff_fast_two_sum(v.hi, fmaf(v.hi, k, v.lo)));
+    return true;
 }
 
 // The d-step by the block that finished last (AIA/aia_cpu.cpp:172-263): reduce
@@ -235,7 +237,19 @@ __global__ void __launch_bounds__(kAiaThreads)
         const ff X = ff_add(ff_add(ff_mul_f(T.adj[0][0], b0), ff_mul_f(T.adj[0][1], b1)), ff_mul_f(T.adj[0][2], b2));
         const ff Y = ff_add(ff_add(ff_mul_f(T.adj[1][0], b0), ff_mul_f(T.adj[1][1], b1)), ff_mul_f(T.adj[1][2], b2));
         ff c, s;  // cos and sin of phi = atan2(-Y, X), X ~ x2, Y ~ x3
-        aia_unit(X, Y, &c, &s);
+        if (!aia_unit(X, Y, &c, &s)) {
+            // an intensity, or a sum of them, is not finite: as 64 bits make it of infinities and NaN
+            const float x = fmaf(T.adj[0][0].hi, b0, fmaf(T.adj[0][1].hi, b1, T.adj[0][2].hi * b2));
+            const float y = fmaf(T.adj[1][0].hi, b0, fmaf(T.adj[1][1].hi, b1, T.adj[1][2].hi * b2));
+            if constexpr (FINAL) {
+                const float p = atan2f(-y, x) + d0.hi;
+                phi[j] = p > 3.14159274f ? p - 6.28318531f : p < -3.14159274f ? p + 6.28318531f : p;
+                continue;
+            } else if (!isinf(x) && !isinf(y)) {  // hypot is NaN, not infinite
+                c = ff{1.f, 0.f};
+                s = ff{0.f, 0.f};
+            }
+        }
         if constexpr (FINAL) {
             // phi + delta_0 in (-pi, pi]: atan2f, corrected by the sine of what it is off
             const float p0 = atan2f(s.hi, c.hi);

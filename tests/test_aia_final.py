@@ -36,3 +36,41 @@ def test_phase_for_given_shifts_is_wrapped(glsu, first):
     assert it == 0
     assert phi.min() >= -np.pi - 1e-6 and phi.max() <= np.pi + 1e-6
     assert np.abs(np.angle(np.exp(1j * (phi - ref)))).max() <= 1e-4
+
+
+def _xy(column, deltas):
+    """The two cofactor sums of one pixel in 64 bits, as IEEE arithmetic gives them (right-hand sides in FP32)."""
+    d = np.asarray(deltas, np.float32).astype(np.float64)
+    c, s = np.cos(d), np.sin(d)
+    a = np.stack([np.ones_like(d), c, s], 1)
+    cof = np.linalg.inv(a.T @ a) * np.linalg.det(a.T @ a)
+    b = [np.float32(0)] * 3
+    for v, ck, sk in zip(column, c.astype(np.float32), s.astype(np.float32)):
+        b = [np.float32(b[0] + v), np.float32(b[1] + v * ck), np.float32(b[2] + v * sk)]
+    return [cof[r, 0] * np.float64(b[0]) + cof[r, 1] * np.float64(b[1]) + cof[r, 2] * np.float64(b[2]) for r in (1, 2)]
+
+
+@pytest.mark.parametrize("frame", [0, 1, 2, 3])
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+def test_pixels_that_are_not_finite(glsu, bad, frame):
+    """Without an iteration such a pixel's phase is what 64-bit arithmetic makes of
+    it (mostly NaN), the others' what it is without it.  With iterations a run ends as
+    not positive definite where the pixel's unit vector is infinity over infinity."""
+    deltas = np.array([0.3, 1.7, 3.3, 4.8])
+    f = _frames(4, 37, 65, deltas)
+    a = glsu.AIA(4, 65, 37)
+    good, _, _, _, _ = a.run(list(f), deltas, max_iter=0)
+    f[frame, 5, 7] = bad
+    phi, _, _, _, _ = a.run(list(f), deltas, max_iter=0)
+    with np.errstate(invalid="ignore"):
+        x, y = _xy(f[:, 5, 7], deltas)
+        want = np.angle(np.exp(1j * (np.arctan2(-y, x) + np.float64(np.float32(deltas[0])))))
+        infinite = np.isinf(np.hypot(x, y))
+    assert np.isnan(phi[5, 7]) if np.isnan(want) else abs(np.angle(np.exp(1j * (phi[5, 7] - want)))) <= 1e-4
+    phi[5, 7] = good[5, 7]
+    assert np.array_equal(phi, good)
+    if infinite:
+        with pytest.raises(glsu.GlsuError) as e:
+            a.run(list(f), deltas, max_iter=5)
+        assert e.value.code == glsu.ERR_NOT_POSDEF
+    a.close()
