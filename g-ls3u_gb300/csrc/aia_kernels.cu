@@ -36,7 +36,8 @@ constexpr int kAiaThreads = 256;
 // [2M+2] status (0 ok, else GLSU_ERR_NOT_POSDEF)
 
 // What the phi-step needs of the shifts: their cosines and sines, and rows 2
-// and 3 of adj(A1), signed by det(A1), as float-float.
+// and 3 of adj(A1), signed by det(A1) and scaled by a power of two so that a row's
+// products with finite sums of intensities stay finite, as float-float.
 struct AiaTables {
     float c[kAiaMaxM], s[kAiaMaxM];
     ff adj[2][3];
@@ -78,7 +79,8 @@ __device__ void aia_tables(const double *__restrict__ state, int M, double *cs, 
         const double det = A[0][0] * (A[1][1] * A[2][2] - A[1][2] * A[2][1]) -
                            A[0][1] * (A[1][0] * A[2][2] - A[1][2] * A[2][0]) +
                            A[0][2] * (A[1][0] * A[2][1] - A[1][1] * A[2][0]);
-        const double sg = det < 0 ? -1.0 : 1.0;
+        const double top = fmax(fmax(fmax(fabs(c10), fabs(c11)), fabs(c12)), fmax(fmax(fabs(c20), fabs(c21)), fabs(c22)));
+        const double sg = ldexp(det < 0 ? -1.0 : 1.0, top > 0 ? -2 - ilogb(top) : 0);
         tab->adj[0][0] = ff_of(sg * c10); tab->adj[0][1] = ff_of(sg * c11); tab->adj[0][2] = ff_of(sg * c12);
         tab->adj[1][0] = ff_of(sg * c20); tab->adj[1][1] = ff_of(sg * c21); tab->adj[1][2] = ff_of(sg * c22);
     }

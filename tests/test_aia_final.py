@@ -74,3 +74,15 @@ def test_pixels_that_are_not_finite(glsu, bad, frame):
             a.run(list(f), deltas, max_iter=5)
         assert e.value.code == glsu.ERR_NOT_POSDEF
     a.close()
+
+
+def test_frames_near_the_range_of_fp32(glsu):
+    """Intensities whose products with the system's cofactors pass FP32's range give
+    the phases of the same frames scaled down (bar of the given shifts' phases)."""
+    deltas = np.array([0.3, 1.7, 3.3, 4.8])
+    f = _frames(4, 37, 65, deltas)
+    a = glsu.AIA(4, 65, 37)
+    small, _, _, _, _ = a.run(list(f), deltas, max_iter=0)
+    large, _, _, _, _ = a.run(list(np.ldexp(f, 118)), deltas, max_iter=0)
+    a.close()
+    assert np.abs(np.angle(np.exp(1j * (small.astype(np.float64) - large)))).max() <= 1e-4
