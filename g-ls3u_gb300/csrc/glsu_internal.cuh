@@ -195,6 +195,7 @@ struct WffPlan {
     int fft64_L = 0;
     void *d_h64 = nullptr;   // nfy x fft64_L real spectra of the modulated windows
     void *d_tw64 = nullptr;  // fft64_L twiddles
+    uint8_t *d_wide64 = nullptr;  // per plane and column: to be done directly
     int init_colfft64();
     bool use_fft64() const { return fft64_L > 0 && d_h64 && d_tw64 && column_method() == GLSU_METHOD_FFT; }
 

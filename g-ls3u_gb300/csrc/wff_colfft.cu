@@ -151,6 +151,8 @@ void WffPlan::release_colfft()
     cudaFree(d_tw);
     cudaFree(d_h64);
     cudaFree(d_tw64);
+    cudaFree(d_wide64);
+    d_wide64 = nullptr;
     d_khat = d_tw = d_h64 = d_tw64 = nullptr;
     fft64_L = 0;
     fft_L = 0;

@@ -52,3 +52,38 @@ def test_explicit_fft_stays_refused_and_env_keeps_direct(glsu, monkeypatch):
     w = glsu.WFF2(64, 256, "f64", p)
     assert w.tuning()["fft_length"] == 0 and w.tuning()["method"] == glsu.METHOD_DIRECT
     w.close()
+
+
+@pytest.mark.parametrize("bad", [1e9, 1e300 ** 0.1, np.inf, np.nan])
+def test_a_pixel_acts_on_its_rows_only(glsu, bad):
+    """One large or non-finite pixel acts on the rows that two column filters connect
+    with it (40: the direct kernel is compiled for half-size 20), as with the direct
+    kernel; elsewhere the field is as without it, and for finite values the whole
+    output is the direct kernel's.  Bar 1e-11 of the output there."""
+    rng = np.random.default_rng(3)
+    h, w = 400, 90
+    y, x = np.mgrid[0:h, 0:w].astype(np.float64)
+    f = np.exp(1j * (0.3 * x - 0.2 * y)) + 0.3 * (rng.standard_normal((h, w)) + 1j * rng.standard_normal((h, w)))
+    p = glsu.WffParams(3.0, -0.4, 0.4, 0.5, HALF / 3.0, -0.5, 0.5, 0.21, 0.1)
+    f[200, 40] = 0
+    a, length = _run(glsu, f, p, False)
+    assert length == 512
+    f[200, 40] = bad
+    b, _ = _run(glsu, f, p, False)
+    d, _ = _run(glsu, f, p, True)
+    far = np.r_[0:200 - 40, 200 + 41:h]
+    assert np.abs(a - b)[far].max() <= 1e-11 * np.abs(a).max()
+    assert np.abs(d - b)[far].max() <= 1e-11 * np.abs(a).max()
+    if np.isfinite(bad):
+        assert (np.abs(d - b).max(1) <= 1e-11 * np.abs(d).max(1)).all()
+
+
+def test_columns_of_a_wide_range(glsu):
+    """Rows from 1 to 2^-40 of the largest in every column: the direct kernel's output, row by row."""
+    y, x = np.mgrid[0:300, 0:70].astype(np.float64)
+    f = np.exp2(-y * 40 / 300) * np.exp(1j * (0.2 * x - 0.1 * y))
+    p = glsu.WffParams(3.0, -0.4, 0.4, 0.5, HALF / 3.0, -0.5, 0.5, 0.21, 0.0)
+    b, length = _run(glsu, f, p, False)
+    assert length == 384
+    d, _ = _run(glsu, f, p, True)
+    assert (np.abs(d - b).max(1) <= 1e-11 * np.abs(d).max(1)).all()
