@@ -264,8 +264,8 @@ int glsu_dpra_update_ref_phi(glsu_dpra *h);
 int glsu_dpra_batch_step(glsu_dpra *const *handles, int n, const void *const *d_frames, int img_type);
 int glsu_dpra_batch_wait(glsu_dpra *const *handles, int n);
 /* Staged batch (no counterpart in the reference): many FP32 plain-form DPRA
- * handles (any sizes, windows and WFF parameters; at most 128 per class and
- * launch, more are split) run one frame each per step, stage by stage: per
+ * handles (any sizes, windows and WFF parameters; at most 64 per class and
+ * launch on the tensor cores, 128 by FFTs, more are split) run one frame each per step, stage by stage: per
  * sequence on its own stream the least squares and the WFF2 row pass; then
  * the column sweeps class by class, a class being the sequences that share a
  * y-filter (tensor-core sweep) or a transform length (FFT sweep), each as one
@@ -276,10 +276,10 @@ int glsu_dpra_batch_wait(glsu_dpra *const *handles, int n);
  * (after its i-th batched frame the reference is updated when i % rr == 0).
  * glsu_dpra_batch_run returns after enqueueing on the batch's stream;
  * d_frames[i] is handle i's device frame (U8 or F32) or NULL when its
- * sequence has ended.  In graph mode (glsu_dpra_batch_set_graph) each step
- * after the first is one CUDA graph launch (one graph per set of active
- * sequences and reference parities, inputs first copied into the handles'
- * frame buffers).  The handles must outlive the batch and are not used
+ * sequence has ended.  In graph mode (glsu_dpra_batch_set_graph) a step whose
+ * set of active sequences and reference parities comes a second time becomes
+ * a CUDA graph, which that and later such steps launch (inputs first copied into
+ * the handles' frame buffers); steps that come once run as without it.  The handles must outlive the batch and are not used
  * elsewhere while it runs. */
 typedef struct glsu_dpra_batch glsu_dpra_batch;
 int glsu_dpra_batch_create(glsu_dpra_batch **out, glsu_dpra *const *handles, int n);
