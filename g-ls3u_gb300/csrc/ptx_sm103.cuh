@@ -84,11 +84,9 @@ __device__ __forceinline__ void tma_load_5d(void *dst, const CUtensorMap *tm, ui
 }
 
 // One lane of a converged warp.  A loop of tcgen05.mma is to run under this
-// and not under lane == 0: the compiler then keeps the instruction's operands
-// in uniform registers, where a data-dependent branch makes it move each of
-// them there before every MMA.  256 MMAs of M = 128, K = 16 back to back, A in
-// TMEM: 110 cycles each under threadIdx.x == 0 whatever N up to 192; 43 at
-// N = 64, 59 at N = 96, 75 at N = 128 under elect.
+// and not under a test of the thread index: 256 MMAs of M = 128, K = 16 back to
+// back, A in TMEM, take 110 cycles each under threadIdx.x == 0 whatever N up to
+// 192; 43 at N = 64, 59 at N = 96, 75 at N = 128 under elect.
 __device__ __forceinline__ bool elect_one()
 {
     uint32_t e;

@@ -294,14 +294,13 @@ __device__ __forceinline__ bool tc_reaches(const TcSeq &q, const unsigned char *
     return sr * sr + si * si >= thr * thr;
 }
 
-// The value of lane 0, which the compiler then knows to be the warp's.
+// The value of lane 0.
 __device__ __forceinline__ int uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
 
 constexpr uint32_t kTcWaitCycles = 1u << 31;
-// Bounded wait, the clock in 32 bits: short, as its copies in every role share the
-// instruction cache with the roles' loops.  After a
-// timeout (ok false) waits return at once: the roles then run to their ends,
-// within their buffers, and the results are not used.
+// Bounded wait, the clock in 32 bits, as its copies in every role count towards the
+// size of the code.  After a timeout (ok false) waits return at once: the roles then
+// run to their ends, within their buffers, and the results are not used.
 __device__ __forceinline__ void wait_ok(uint64_t *bar, uint32_t parity, bool &ok)
 {
     if (!ok) return;
@@ -376,7 +375,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     float(*kcol)[kCols] = reinterpret_cast<float(*)[kCols]>(tb + kMaxTapBytes + 768);  // of two tiles, in turns
     float(*kmax)[kCols] = kcol + 2, (*kmin)[kCols] = kcol + 4;  // by the two warpgroups that scale
 
-    // warp-uniform to the compiler too: the operands of the tcgen05 instructions derive from it
+    // by a shuffle, as everything that the operands of the tcgen05 instructions derive from
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31, wg = warp >> 2, w4 = warp & 3;
     const int nchunks = (RW + 16 * m + kChunkRows - 1) / kChunkRows;
     int nitems = nitems_full, listn = 0;
@@ -763,8 +762,8 @@ __global__ void __launch_bounds__(kThreads, 1)
                         }
                         __syncwarp();
                     };
-                    // one body for both halves: every SM sub-partition runs all roles, and their loops have to
-                    // fit the instruction cache together (a 1024^2 frame by the kernel's size in KB: 58 1.75 ms,
+                    // one body for both halves: every SM sub-partition runs all roles, and the time follows the
+                    // size of their code together (a 1024^2 frame by the kernel's size in KB: 60 1.75 ms,
                     // 71 1.79, 77 1.92, 84 2.17)
 #pragma unroll 1
                     for (int hb = 0; hb < 2 && 2 * i + hb < nb; hb++) {
