@@ -243,8 +243,9 @@ int launch_colfft_batch(const WffPlan *const *plans, int n, cudaStream_t s)
 // Timed search.  Candidates: the direct column kernel, and the FFT sweep at
 // the two shortest compiled transform lengths, then, at the faster length,
 // with the other compiled CTA width, and the tensor-core sweep.  Each is launched once (warm-up), then
-// twice between CUDA events on the plan's own buffers; the kernels have no
-// data-dependent control flow, so the buffers' contents do not matter.  The
+// twice between CUDA events on the plan's own buffers.  Only the tensor-core sweep's
+// time depends on what they hold (its FP64 decisions, 4% of a frame, and the columns
+// it does again, of which zeroed buffers have none).  The
 // FFT is taken only when at least 10% faster than the direct kernel, so
 // that near ties keep the direct kernel.  Results are kept per shape for the
 // process, so every handle of a shape runs the same kernels.
@@ -278,8 +279,9 @@ constexpr double kModelLaunchMs = 0.05;
 // Direct kernel: per output pixel, x-frequency and y-frequency, two column
 // filters of 2S+1 taps (S the instantiated half-size), the first one also
 // over the 2S-row halo of each 128-row tile, at a rate per instantiation.
-// FFT sweep: per column and x-frequency, 2 nfy + 2 transforms of length L
-// in a number of radix passes.
+// FFT sweep (colfft_model_ms): per column and x-frequency, 2 nfy + 2 transforms of
+// length L in a number of radix passes.  Where the tensor-core sweep takes its place,
+// that one's model (tc_model_ms).
 double WffPlan::colfft_model_ms() const
 {
     const double units = (double)pitch * nfx * fft_L * (fft_nst * (2.0 * nfy + 2.0) + kModelFftColumnUnits);
@@ -306,8 +308,8 @@ bool WffPlan::local_sweep() const
     return !unit_input && d_tctaps && colfft_model_ms() >= 0.9 * model_ms(GLSU_METHOD_DIRECT);
 }
 
-// AUTO without timing: the shortest compiled transform length (built by
-// init_colfft), its default CTA width, and the FFT sweep when its modelled
+// AUTO without timing: the shortest compiled transform length, its default CTA
+// width, and the sweep of GLSU_METHOD_FFT (tensor cores or FFTs) when its modelled
 // time is below 0.9 x the direct kernel's.
 int WffPlan::choose_by_model()
 {

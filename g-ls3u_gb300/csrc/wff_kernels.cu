@@ -765,10 +765,10 @@ static TileMask with_margins(TileMask m, int my, int mx)
 
 // Planes per CTA of the row passes.  A frame has (pitch/128) x (H/32) row
 // tiles, 16 at 256 x 256: below one wave (two CTAs per SM) the planes are
-// dealt out over blockIdx.z to fill it.  Both row passes of a 256 x 256 frame
-// with sigma 20 and 7 x 7 frequencies: 164 -> 60 us; the 480 x 640, sigma 10
-// frame 721 -> 593 us in all.  At 1024^2 (256 tiles) four CTAs per SM
-// instead of the unsplit pass made the frame 30 us slower.
+// dealt out over blockIdx.z to fill it.  Both row passes by the stage events: 256 x 256
+// with sigma 20 and 7 x 7 frequencies 136 -> 38 us, 480 x 640 with sigma 10 and 21 x 21
+// 244 -> 113 us.  At 1024^2 (256 tiles) four CTAs per SM instead of the unsplit pass
+// made the frame 30 us slower.
 static int rows_zplanes(const WffPlan &P)
 {
     const int tiles = (P.pitch / kRowTileCols) * ((P.H + kRowTileRows - 1) / kRowTileRows);

@@ -41,12 +41,12 @@
 // each accumulator sees the same K steps in the same order whatever the tile:
 // a row's bits do not depend on the tile height, the batch or a tile mask.
 //
-// Bound: the waits between the stages, and instruction issue.  At 1024^2, sigma
-// 10, 21 x 21 frequencies the sweep takes 1.40 ms (the FFT sweep 3.18): 2.8
-// instructions a clock per SM, about 170 per 16 x 64 block, wy and pass for the
-// splitting and thresholding, a quarter of them waiting.  With nearly all of A's,
-// B's and C's arithmetic taken out 1.0 of 1.39 ms is left: the chain slot, MMAs,
-// commit, next slot.  A third A warpgroup, up to four A1 slots, filling a slot in
+// Bound: instruction issue, and the waits between the stages.  At 1024^2, sigma
+// 10, 21 x 21 frequencies the sweep takes 1.50 ms (the FFT sweep 3.18): 3.0
+// instructions a clock per SM, 76% of the issue slots, about 170 per 16 x 64 block, wy
+// and pass for the splitting and thresholding, a quarter of them waiting; tensor pipe
+// 30%.  In an earlier form of 1.39 ms, with nearly all of A's, B's and C's arithmetic
+// taken out 1.0 was left: the chain slot, MMAs, commit, next slot.  A third A warpgroup, up to four A1 slots, filling a slot in
 // halves, skipping empty blocks and sleeping waits each left the time as it was
 // or made it longer.  The MMAs alone would take 0.5 ms (N/2 cycles each at M =
 // 128, K = 16, A in TMEM); the DRAM is at 3%.
@@ -1086,8 +1086,12 @@ int tc_pass_grain(const double *gy, int s, double &shrink)
 }
 
 // Modelled cost of a sweep of these plans with 32 rb-row tiles, in steps of
-// the busiest SM: tiles are dealt out round robin, so a few tiles more than
-// the SMs cost a whole round.
+// the busiest SM: half whole rounds of mean tiles (tiles are dealt out round robin, so
+// a few more than the SMs cost a round), half an even share, as tiles at the image's
+// ends are short and let their SM go ahead.  Over nine shapes (200 x 300 to 1024^2,
+// sigma 5 to 15) the height with the least cost took the least time of 5, 4 and 2 or
+// up to 2% more: 1024^2, sigma 10 1503, 1556 and 2183 us; 256^2 184, 178 and 190;
+// 733 x 1021, sigma 7 418, 459 and 575; 384 x 512 356, 348 and 427 with equal costs.
 double tc_cost(const WffPlan *const *plans, int n, int rb, int sms)
 {
     double total = 0, items = 0, mx = 0;
@@ -1239,7 +1243,8 @@ void WffPlan::release_tc()
 }
 
 // Modelled time (ms): the steps of the busiest SM at 250 cycles each (measured
-// 247 at sigma 10 and 241 at sigma 15 on large frames), plus launch and tail.
+// 265 at sigma 10 and 15 on large frames: 1.38 ms modelled at 1024^2, 1.50 measured),
+// plus launch and tail.
 double tc_model_ms(const WffPlan &P)
 {
     int rb[4];

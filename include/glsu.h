@@ -59,9 +59,16 @@ extern "C" {
  * convolution in the frequency domain of each column with shared-memory
  * transforms.  AUTO (the default) picks one of the two from
  * the handle's shape with a cost model of both kernels, so the choice, and
- * therefore every output bit, is the same in every process.  TIMED picks
+ * therefore every output bit, is the same in every process; FP64 handles have
+ * a column FFT of their own under AUTO.  TIMED picks
  * the one measured fastest on this GPU (glsu_wff_tuning); its choice can
- * differ from run to run where the two are close. */
+ * differ from run to run where the two are close.
+ * How far one pixel far above the rest, or not finite, acts: DIRECT, and AUTO
+ * for FP64 and for the windows where it would take DIRECT before FFTs: on the
+ * rows and columns that the filters connect with it.  Tensor cores beyond that:
+ * also, with 2^-40 of its size, on the other rows (at most 160 and the filters'
+ * halo) of its tile, and a non-finite one on up to 15 rows more.  FFTs: on
+ * whole columns, with 2^-24 of its size. */
 #define GLSU_METHOD_AUTO 0
 #define GLSU_METHOD_DIRECT 1
 #define GLSU_METHOD_FFT 2
@@ -147,7 +154,7 @@ int glsu_wff_set_method(glsu_wff *h, int method);
  * windows run the direct kernel. */
 typedef struct {
     int method;          /* GLSU_METHOD_DIRECT or GLSU_METHOD_FFT: the sweep that runs */
-    int fft_length;      /* transform length of the FFT plan (0: no FFT plan) */
+    int fft_length;      /* transform length of the FFT plan (0: no FFT plan), also where the tensor cores run */
     int fft_columns;     /* columns per CTA of the FFT sweep */
     int fft_radix_order; /* radix order of the FFT passes (always 0) */
     int tuned;           /* 0: not resolved; 1: resolved by timing; 2: by the cost model */
