@@ -64,11 +64,11 @@ extern "C" {
  * the one measured fastest on this GPU (glsu_wff_tuning); its choice can
  * differ from run to run where the two are close.
  * How far one pixel far above the rest, or not finite, acts: DIRECT, and AUTO
- * for FP64 and for the windows where it would take DIRECT before FFTs: on the
- * rows and columns that the filters connect with it.  Tensor cores beyond that:
- * also, with 2^-40 of its size, on the other rows (at most 160 and the filters'
- * halo) of its tile, and a non-finite one on up to 15 rows more.  FFTs: on
- * whole columns, with 2^-24 of its size. */
+ * for FP64 and (WFF2 handles) for the windows where it would take DIRECT before
+ * FFTs: on the rows and columns that the filters connect with it.  Tensor cores
+ * otherwise: also, with 2^-40 of its size, on the other rows (at most 160 and the
+ * filters' halo) of its tile; a non-finite one on up to 15 rows more.  FP32 FFTs:
+ * on whole columns, with 2^-24 of its size. */
 #define GLSU_METHOD_AUTO 0
 #define GLSU_METHOD_DIRECT 1
 #define GLSU_METHOD_FFT 2
