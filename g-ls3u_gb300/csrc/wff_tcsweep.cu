@@ -491,24 +491,25 @@ __global__ void __launch_bounds__(kThreads, 1)
                         int taken = 0, done = 0;  // pairs of blocks
                         for (int st = from; st < to; st += 2, n++) {
                             const uint32_t slot = n & 1;
-                            warp_wait(&afull[slot], (n >> 1) & 1, ok);
                             const int nst = min(2, to - st), top = min(st + nst - 1 + W - b0, nb);
+                            uint32_t d[2], off[2], id[2];
+#pragma unroll
+                            for (int h = 0; h < 2; h++) {
+                                const int lo = max(st + h - b0, 0), hi = min(st + h + W - b0, nb);
+                                off[h] = (uint32_t)(lo + b0 - st - h) * 32;  // 16 outputs: 512 bytes
+                                d[h] = tD + 16 * lo;
+                                id[h] = idesc | ((uint32_t)(hi - lo) << 18);
+                            }
                             for (; 2 * taken < top; taken++)
                                 if ((used >> taken) & 1) warp_wait(&fre[taken], ((parity >> taken) & 1) ^ 1, ok);
+                            warp_wait(&afull[slot], (n >> 1) & 1, ok);
                             tc_fence_after();
                             // the small products of both steps, then the large ones
-#pragma unroll
-                            for (int part = 0; part < 2; part++)
-#pragma unroll
-                                for (int h = 0; h < 2; h++) {
-                                    if (h == 1 && nst < 2) break;
-                                    const int lo = max(st + h - b0, 0), hi = min(st + h + W - b0, nb);
-                                    const uint32_t off = (uint32_t)(lo + b0 - st - h) * 32;  // 16 outputs: 512 bytes
-                                    const uint32_t d = tD + 16 * lo, a = tA + 32 * slot + 16 * h;
-                                    const uint32_t id = idesc | ((uint32_t)(hi - lo) << 18);
-                                    if (part == 0) umma_cross(d, a, bhi + off, blo + off, id);
-                                    else umma_main(d, a, bhi + off, id);
-                                }
+                            const uint32_t a = tA + 32 * slot;
+                            umma_cross(d[0], a, bhi + off[0], blo + off[0], id[0]);
+                            if (nst > 1) umma_cross(d[1], a + 16, bhi + off[1], blo + off[1], id[1]);
+                            umma_main(d[0], a, bhi + off[0], id[0]);
+                            if (nst > 1) umma_main(d[1], a + 16, bhi + off[1], id[1]);
                             umma_commit_warp(&afree[slot]);
                             // pairs with all their products
                             const int fin = st + 2 < to ? min(st + 2 - b0, nb) : nb;
@@ -991,7 +992,7 @@ void tap_parts(double g, int grain, __half &hi, __half &lo)
 // better of two grains is taken (-5 keeps the largest tap within 11 bits).  Data: real
 // parts of waves from the window's centre frequency to 1.2 / sigma off it, without and
 // with noise, amplitudes over a power of two.  Bit patterns instead of half and math
-// functions, as this runs at a handle's creation (half-size 30: 2.4 ms, 48: 3.6; with the library's conversions 6.5 and 10).
+// functions, as this runs at a handle's creation (half-size 30: 1.3 ms, 48: 1.9).
 int tc_pass_grain(const double *gy, int s, double &shrink)
 {
     constexpr int kGrains = 2, kGrain[kGrains] = {-4, -5};
@@ -1029,7 +1030,7 @@ int tc_pass_grain(const double *gy, int s, double &shrink)
         return (double)(rng >> 11) * 0x1p-53;
     };
     double ee = 0, er[kGrains] = {}, rr[kGrains] = {};  // sums of exact^2, exact x loss, loss^2
-    for (int n = 0; n < 768; n++) {
+    for (int n = 0; n < 384; n++) {
         const int off = n & 15, kind = (n >> 4) & 7, steps = (off + taps + 15) / 16;
         const double amp = std::exp2(9 + uniform()), phase = 2 * M_PI * uniform();
         const double slope = 0.4 * (kind & 3) * 3.0 / std::max(s, 1), noise = kind & 4 ? 4.0 : 0.0;
