@@ -1404,9 +1404,8 @@ extern "C" int glsu_dpra_batch_run(glsu_dpra_batch *b, const void *const *d_fram
             c = glsu_dpra_batch::Graph();
             c.key = key;
         }
-    }
-    if (g) {
-        // the graph reads each handle's own frame buffer: copy the inputs in
+        // a graph reads each handle's own frame buffer, and so does a step that is not captured yet: copy the
+        // inputs in (the caller's buffers are free again once the step has begun)
         for (size_t i = 0; i < n; i++) {
             glsu_dpra *h = b->h[i];
             if (!active[i]) continue;
@@ -1414,6 +1413,8 @@ extern "C" int glsu_dpra_batch_run(glsu_dpra_batch *b, const void *const *d_fram
                                           cudaMemcpyDeviceToDevice, b->stream));
             in[i] = h->d_img;
         }
+    }
+    if (g) {
         if (!g->exec) {
             GLSU_CUDA_TRY(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
             const int rc = batch_enqueue(b, active, in, img_type);

@@ -285,8 +285,9 @@ int glsu_dpra_batch_wait(glsu_dpra *const *handles, int n);
  * d_frames[i] is handle i's device frame (U8 or F32) or NULL when its
  * sequence has ended.  In graph mode (glsu_dpra_batch_set_graph) a step whose
  * set of active sequences and reference parities comes a second time becomes
- * a CUDA graph, which that and later such steps launch (inputs first copied into
- * the handles' frame buffers); steps that come once run as without it.  The handles must outlive the batch and are not used
+ * a CUDA graph, which that and later such steps launch; steps that come once run
+ * as without it.  Each step after the first copies its inputs into the handles'
+ * frame buffers before all else.  The handles must outlive the batch and are not used
  * elsewhere while it runs. */
 typedef struct glsu_dpra_batch glsu_dpra_batch;
 int glsu_dpra_batch_create(glsu_dpra_batch **out, glsu_dpra *const *handles, int n);
