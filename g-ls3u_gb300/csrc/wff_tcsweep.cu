@@ -42,7 +42,7 @@
 // a row's bits do not depend on the tile height, the batch or a tile mask.
 //
 // Bound: instruction issue, and the waits between the stages.  At 1024^2, sigma
-// 10, 21 x 21 frequencies the sweep takes 1.50 ms (the FFT sweep 3.18): 3.0
+// 10, 21 x 21 frequencies the sweep takes 1.49 ms (the FFT sweep 3.18): 3.0
 // instructions a clock per SM, 76% of the issue slots, about 170 per 16 x 64 block, wy
 // and pass for the splitting and thresholding, a quarter of them waiting; tensor pipe
 // 30%.  In an earlier form of 1.39 ms, with nearly all of A's, B's and C's arithmetic
