@@ -884,74 +884,139 @@ __global__ void __launch_bounds__(kThreads, 1)
 // The wide columns of a tile once more, directly in FP32 from R, as the direct
 // column kernel does them: a value then acts on the 2s rows around it only.  Runs
 // where AUTO would take the direct kernel but for this file (WffPlan::tc_local) and
-// the input is not of unit modulus.  One CTA a tile; with no wide column, the rule on
-// measured fields, it costs its launch.
-constexpr int kLocalThreads = 256;
-__global__ void __launch_bounds__(kLocalThreads) wff_tc_local_kernel(const __grid_constant__ TcTable<1> tab, int nitems,
+// the input is not of unit modulus.  With no wide column, the rule on measured fields,
+// it costs its launch.  A CTA takes four wide columns of a tile at a time, 64 threads
+// each, four rows a thread (eight FMAs for a tap and a value read from shared memory).
+// Whole calls, one pixel of 1e12 (direct kernel): 512 x 512 with sigma 3 0.40 ms (0.46),
+// 733 x 1021 with sigma 5 0.77 (1.35); every column wide: 1.54 (0.46) and 2.65 (1.35),
+// 2.85 and 5.05 with a column at a time and a row a thread.
+constexpr int kLocalCols = 4, kLocalThreads = 64 * kLocalCols;
+
+// Element i of D and T stands at local_at(i): threads four rows apart then meet no bank twice.
+__device__ __forceinline__ int local_at(int i) { return i + (i >> 2); }
+
+// Four outputs i0 .. i0 + 3, i0 = 4 lt, of sum_j g[j] v[i + j], j = 0 .. 2s; taps beyond the window do not
+// meet a value (0 times NaN), and v is readable to i0 + 2s + 3.
+__device__ __forceinline__ void local_filter4(const float *g, const float2 *v, int s, int lt, float2 (&u)[4])
+{
+    v += 5 * lt;
+#pragma unroll
+    for (int r = 0; r < 4; r++) u[r] = make_float2(0.f, 0.f);
+    const auto edge = [&](int j) {
+        const float2 x = v[local_at(j)];
+#pragma unroll
+        for (int r = 0; r < 4; r++)
+            if (j >= r && j - r <= 2 * s) u[r] = make_float2(fmaf(g[j - r], x.x, u[r].x), fmaf(g[j - r], x.y, u[r].y));
+    };
+    for (int j = 0; j < 3; j++) edge(j);
+    if (s < 2) {
+        for (int j = 3; j < 2 * s + 4; j++) edge(j);
+        return;
+    }
+    float t1 = g[2], t2 = g[1], t3 = g[0];
+#pragma unroll 4
+    for (int j = 3; j <= 2 * s; j++) {
+        const float2 x = v[local_at(j)];
+        const float t0 = g[j];
+        u[0] = make_float2(fmaf(t0, x.x, u[0].x), fmaf(t0, x.y, u[0].y));
+        u[1] = make_float2(fmaf(t1, x.x, u[1].x), fmaf(t1, x.y, u[1].y));
+        u[2] = make_float2(fmaf(t2, x.x, u[2].x), fmaf(t2, x.y, u[2].y));
+        u[3] = make_float2(fmaf(t3, x.x, u[3].x), fmaf(t3, x.y, u[3].y));
+        t3 = t2;
+        t2 = t1;
+        t1 = t0;
+    }
+    for (int j = 2 * s + 1; j < 2 * s + 4; j++) edge(j);
+}
+
+__global__ void __launch_bounds__(kLocalThreads, 4) wff_tc_local_kernel(const __grid_constant__ TcTable<1> tab, int nitems,
                                                                      int s, int m, int rw,
                                                                      const __grid_constant__ Taps<float, 60> gA,
                                                                      const __grid_constant__ Taps<float, 60> gB)
 {
-    __shared__ float2 D[kMaxChunks * kChunkRows], T[kMaxChunks * kChunkRows];
+    constexpr int kRows = kMaxChunks * kChunkRows + 4, kRowsT = 260 + 2 * kMaxTcHalf;
+    __shared__ float2 Rc[kLocalCols][kRows], D[kLocalCols][kRows + kRows / 4], T[kLocalCols][kRowsT + kRowsT / 4];
     __shared__ float a[2 * kMaxTcHalf + 1], b[2 * kMaxTcHalf + 1];
-    __shared__ uint8_t wide[kCols];
     const TcSeq &q = tab.seq[0];
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, grp = tid >> 6, lt = tid & 63;
     for (int j = tid; j <= 2 * s; j += kLocalThreads) {
         a[j] = gA.g[60 - s + j];
         b[j] = gB.g[60 - s + j];
     }
     const float thr = *q.thr, thr2 = thr * thr;
     const int pairs = (q.H + 1) >> 1;
-    for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
-        __syncthreads();
-        if (tid < kCols) wide[tid] = q.wide[(size_t)item * kCols + tid];
-        if (!__syncthreads_or(tid < kCols && wide[tid])) continue;
-        TcTile t;
-        tc_item<1>(tab, 1, item, nullptr, 0, s, m, rw, t);
-        const int y1 = min(t.y0 + rw, q.H), nu = y1 - t.y0 + 2 * s, nr = nu + 2 * s;
-        for (int c = 0; c < kCols && t.x0 + c < q.W; c++) {
-            if (!wide[c]) continue;
-            const float *R = q.R + ((size_t)t.plane * pairs * q.pitch + t.x0 + c) * 4;
-            float2 acc = make_float2(0.f, 0.f);  // of row t.y0 + tid: rw <= kLocalThreads
-            for (int k = 0; k < q.nfy; k++) {
-                const float *P = reinterpret_cast<const float *>(q.ey2 + (size_t)k * q.eys2 + kTcPad);
-                for (int i = tid; i < nr; i += kLocalThreads) {
+    constexpr int kLook = kLocalThreads / 16;  // items whose 64 flags are looked at together
+    for (int first = blockIdx.x; first < nitems; first += kLook * gridDim.x) {
+        const int mine = first + (tid >> 4) * gridDim.x;
+        const bool some =
+            mine < nitems && reinterpret_cast<const uint32_t *>(q.wide)[(size_t)mine * (kCols / 4) + (tid & 15)];
+        if (!__syncthreads_or(some)) continue;
+        for (int item = first, n = 0; n < kLook && item < nitems; n++, item += gridDim.x) {
+            const uint8_t *flag = q.wide + (size_t)item * kCols + (tid & 31);
+            // the same in every warp
+            uint64_t todo = __ballot_sync(0xffffffffu, flag[0]) | (uint64_t)__ballot_sync(0xffffffffu, flag[32]) << 32;
+            if (!todo) continue;
+            TcTile t;
+            tc_item<1>(tab, 1, item, nullptr, 0, s, m, rw, t);
+            if (q.W - t.x0 < kCols) todo &= (1ull << (q.W - t.x0)) - 1;
+            const int y1 = min(t.y0 + rw, q.H), nu = y1 - t.y0 + 2 * s, nr = nu + 2 * s;
+            while (todo) {
+                int c = -1;  // the group's column
+                for (int g = 0; g < kLocalCols; g++) {
+                    if (g == grp && todo) c = __ffsll((long long)todo) - 1;
+                    todo &= todo - 1;
+                }
+                const float *R = q.R + ((size_t)t.plane * pairs * q.pitch + t.x0 + max(c, 0)) * 4;
+                for (int i = lt; i < nr + 3 && c >= 0; i += 64) {
                     const int y = t.y0 - 2 * s + i;
-                    float2 d = make_float2(0.f, 0.f);
-                    if ((unsigned)y < (unsigned)q.H) {
-                        const float *e = R + (size_t)(y >> 1) * q.pitch * 4 + (y & 1), *p = P + (y >> 1) * 4 + (y & 1);
-                        d = make_float2(e[0] * p[0] - e[2] * p[2], e[0] * p[2] + e[2] * p[0]);
+                    const float *e = R + (size_t)(y >> 1) * q.pitch * 4 + (y & 1);
+                    Rc[grp][i] = (unsigned)y < (unsigned)q.H && i < nr ? make_float2(e[0], e[2]) : make_float2(0.f, 0.f);
+                }
+                float2 acc[4];  // of rows t.y0 + 4 lt ..: rw <= 256
+#pragma unroll
+                for (int r = 0; r < 4; r++) acc[r] = make_float2(0.f, 0.f);
+                for (int k = 0; k < q.nfy; k++) {
+                    const float *P = reinterpret_cast<const float *>(q.ey2 + (size_t)k * q.eys2 + kTcPad);
+                    for (int i = lt; i < nr + 3 && c >= 0; i += 64) {
+                        // rows outside the image are zeros times some row's phasor
+                        const int y = min(max(t.y0 - 2 * s + i, 0), q.H - 1);
+                        const float *p = P + (y >> 1) * 4 + (y & 1);
+                        const float2 r = Rc[grp][i];
+                        D[grp][local_at(i)] = make_float2(r.x * p[0] - r.y * p[2], r.x * p[2] + r.y * p[0]);
                     }
-                    D[i] = d;
+                    __syncthreads();
+                    if (c >= 0 && 4 * lt < nu) {
+                        float2 u[4];
+                        local_filter4(a, D[grp], s, lt, u);
+#pragma unroll
+                        for (int r = 0; r < 4; r++) {
+                            const int i = 4 * lt + r, y = t.y0 - s + i;
+                            const bool keep = i < nu && (unsigned)y < (unsigned)q.H &&
+                                              u[r].x * u[r].x + u[r].y * u[r].y >= thr2;
+                            T[grp][local_at(i)] = keep ? u[r] : make_float2(0.f, 0.f);
+                        }
+                    }
+                    __syncthreads();
+                    if (c >= 0 && t.y0 + 4 * lt < y1) {
+                        float2 v[4];
+                        local_filter4(b, T[grp], s, lt, v);
+#pragma unroll
+                        for (int r = 0; r < 4; r++) {
+                            const int y = min(t.y0 + 4 * lt + r, q.H - 1);
+                            const float *p = P + (y >> 1) * 4 + (y & 1);
+                            acc[r].x += p[0] * v[r].x + p[2] * v[r].y;
+                            acc[r].y += p[0] * v[r].y - p[2] * v[r].x;
+                        }
+                    }
                 }
                 __syncthreads();
-                for (int i = tid; i < nu; i += kLocalThreads) {
-                    const int y = t.y0 - s + i;
-                    float2 u = make_float2(0.f, 0.f);
-                    for (int j = 0; j <= 2 * s; j++) {
-                        u.x = fmaf(a[j], D[i + j].x, u.x);
-                        u.y = fmaf(a[j], D[i + j].y, u.y);
+                if (c >= 0)
+#pragma unroll
+                    for (int r = 0; r < 4; r++) {
+                        const int y = t.y0 + 4 * lt + r;
+                        if (y < y1) q.C[(size_t)t.plane * q.H * q.pitch + (size_t)y * q.pitch + t.x0 + c] = acc[r];
                     }
-                    const bool keep = (unsigned)y < (unsigned)q.H && u.x * u.x + u.y * u.y >= thr2;
-                    T[i] = keep ? u : make_float2(0.f, 0.f);
-                }
-                __syncthreads();
-                if (t.y0 + tid < y1) {
-                    const int y = t.y0 + tid;
-                    float2 v = make_float2(0.f, 0.f);
-                    for (int j = 0; j <= 2 * s; j++) {
-                        v.x = fmaf(b[j], T[tid + j].x, v.x);
-                        v.y = fmaf(b[j], T[tid + j].y, v.y);
-                    }
-                    const float *p = P + (y >> 1) * 4 + (y & 1);
-                    acc.x += p[0] * v.x + p[2] * v.y;
-                    acc.y += p[0] * v.y - p[2] * v.x;
-                }
             }
-            __syncthreads();
-            if (t.y0 + tid < y1)
-                q.C[(size_t)t.plane * q.H * q.pitch + (size_t)(t.y0 + tid) * q.pitch + t.x0 + c] = acc;
         }
     }
 }
@@ -1281,7 +1346,7 @@ int launch_tc_sweep(const WffPlan *const *plans, int n, cudaStream_t s)
             const int items = tiles * P.nfx;
             GLSU_TRY(tc_launch_one(rb, tab, items, std::min(items, sms), P, nullptr, nullptr, s));
             if (!tab.seq[0].wide) return GLSU_OK;
-            wff_tc_local_kernel<<<std::min(items, 2 * sms), kLocalThreads, 0, s>>>(
+            wff_tc_local_kernel<<<std::min(items, 4 * sms), kLocalThreads, 0, s>>>(
                 tab, items, P.sy, (P.sy + 3) / 4, 32 * rb, make_taps<float, 60>(P.gy, P.sy, P.inv_norm),
                 make_taps<float, 60>(P.gy, P.sy, 1.0));
             GLSU_CUDA_TRY(cudaGetLastError());
